@@ -364,7 +364,7 @@ def run_b200(args):
                     "nconv": nconv, "reason": reason, "max_rel_residual": max(resid) if resid else None},
                 "roofline": {"kernel": ("rb_spmm_kernel (row-major block SpMV with the fused Chebyshev three-term "
                                         "update, FP32 and FP64 phases)"
-                                        if mixed else "gs_pass_kernel (fused CGS update+dot, DGKS on device)"),
+                                        if mixed else "gs_column_kernel (fused CGS update+dot, DGKS on device)"),
                              "bound": "hbm",
                              "achieved": gs_gbs, "peak": peak, "unit": "GB/s",
                              "frac": (gs_gbs / peak) if gs_gbs else None,

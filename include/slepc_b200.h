@@ -236,7 +236,7 @@ b200_status b200_bv_mult_inplace_trans(b200_bv bv, const double *Q_host, int ldq
  * CGS + DGKS passes.  H_dev (device, j+1 doubles) receives the coefficients
  * and then the norm; norm and lindep (host, nullable) are read back, so the
  * call synchronises the stream.  All working memory comes from one fixed
- * array of about 330 KB compiled into the library, which every GPU that
+ * array of about 660 KB compiled into the library, which every GPU that
  * loads the library holds until the process exits; j at most 253, otherwise
  * B200_ERR_ARG.  The first call on a device (and in each context of it the
  * caller makes current) looks the array's address up and should come before

@@ -25,7 +25,7 @@ enum DeviceError : int {
   kDevErrNonFinite = 4,      // NaN or Inf met in a reduction
 };
 
-// Gram-Schmidt pass actions (bitmask), decided on the device.
+// Gram-Schmidt pass actions (bitmask), decided on the device between passes.
 enum GsAction : int {
   kActNone = 0,
   kActUpdate = 1,   // w <- w - V(:,0:j) coef
@@ -40,32 +40,18 @@ enum GsStage : int {
   kStageDone = 2,
 };
 
-// Per-BV device control block for one column orthogonalisation.  Written by
-// the host before the first pass, then advanced on the device by the last
-// CTA of every Gram-Schmidt pass.
+// Per-BV device control block: the outcome of the last column orthogonalisation and the counters of
+// the run it belongs to.  Written by the Gram-Schmidt kernel; the error bits stay until the host has
+// read them and resets the block.
 struct GsState {
-  int action;        // GsAction bits for the next pass kernel
-  int stage;         // GsStage
-  int pass;          // CGS passes applied so far (1..3)
-  int j;             // column being orthogonalised (columns 0..j-1 are the basis)
-  int normalize;     // 1: scale the result by 1/norm (BVOrthonormalizeColumn)
-  int want_self;     // 1: include w^T w in the dot (column variant); 0: vector variant
-  int lindep;        // linear dependence flag of the last finished column
-  int halt;          // set when a Lanczos run broke down: later steps are skipped
-  int halt_step;     // Lanczos step index at which the breakdown happened
-  int err;           // DeviceError bits
-  int lanczos_step;  // index j of the Lanczos step in flight (for T output)
-  int t_base;        // offset of T output, -1 = none
-  unsigned int ticket;  // CTA arrival counter of the running pass
-  int pad0;
-  double eta;        // DGKS threshold (0.7071)
-  double deftol;     // 10*eps for BV_SafeSqrt
-  double onrm, nrm;  // norms of the current pass
-  double scale;      // multiplier applied by the kScale action
-  double beta_out;   // norm returned to the caller (BVOrthonormalizeColumn's norm)
-  unsigned long long bytes;  // algorithmic bytes moved by the passes since the reset
-  int passes;        // pass kernels that did work since the reset
-  int pad1;
+  unsigned int ticket;  // word of the grid barrier (its top bit flips once per barrier)
+  int lindep;           // linear dependence flag of the last finished column
+  int halt;             // set when a Lanczos run broke down: later steps are skipped
+  int halt_step;        // Lanczos step index at which the breakdown happened
+  int err;              // DeviceError bits
+  int passes;           // passes done since the start of the run
+  double beta_out;      // norm returned to the caller (BVOrthonormalizeColumn's norm)
+  unsigned long long bytes;  // algorithmic bytes moved by those passes
 };
 
 }  // namespace b200

@@ -1,4 +1,4 @@
-// Fused classical Gram-Schmidt with DGKS refinement for sm_100a.
+// Fused classical Gram-Schmidt with DGKS refinement for sm_100a: one cooperative launch per column.
 //
 // Replaces the BV Gram-Schmidt path of SLEPc:
 //   BVOrthogonalizeGS (src/sys/classes/bv/interface/bvorthog.c:145-217)
@@ -8,24 +8,16 @@
 // whose GPU form (bvcuda.cu:204-264, 45-60, 420-548) issues a cuBLAS gemv per
 // half-pass plus 2-4 synchronous device-to-host scalar copies per pass.
 //
-// Here one kernel, gs_pass_kernel, performs any combination of
-//   UPDATE  w <- w - V(:,0:jb) coef      (the second half of CGS pass p)
-//   SCALE   w <- w * scale               (BVOrthonormalizeColumn's 1/norm)
-//   DOT     c <- [V(:,0:jb) w', w'^T w'] (the first half of CGS pass p+1)
-// in one streaming read of V: each CTA of a persistent grid (one per SM)
-// pulls row chunks of all jb columns plus w into shared memory with
-// cp.async.bulk copies completing on an mbarrier (two stages, so the next
-// chunk is in flight while the current one is computed), applies the update
-// row-wise and the dot column-wise from shared memory, and accumulates
-// per-CTA column sums.  The last CTA to finish (atomic ticket) reduces the
-// per-CTA sums in a fixed order (deterministic result), then runs the DGKS
-// decision of BVOrthogonalizeGS on the device and writes the action of the
-// next pass.  The host enqueues a fixed sequence of passes without waiting;
-// passes the device decides against return immediately.
-//
-// A CGS pass of the reference reads V twice (dot, then update); fusing the
-// update of pass p with the dot of pass p+1 reads V three times per column
-// with one DGKS refinement instead of four, and no host round trip.
+// gs_column_kernel runs every pass of a column.  A pass is any combination of
+//   UPDATE  w <- w - V(:,0:jb) coef        (the second half of CGS pass p)
+//   SCALE   w <- w * scale                 (BVOrthonormalizeColumn's 1/norm)
+//   DOT     c <- [V(:,0:jb)^T w', w'^T w'] (the first half of CGS pass p+1)
+// in one streaming read of V; fusing the update of pass p with the dot of pass
+// p+1 reads V three times for a column refined once, where a gemv per half-pass
+// reads it four times.  After a DOT the CTAs meet at a grid barrier, every CTA
+// sums the per-CTA dots in the same fixed order and takes the DGKS decision of
+// BVOrthogonalizeGS for itself (the same bits everywhere), so the next pass
+// starts without a launch and without another exchange.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -35,20 +27,12 @@
 namespace b200 {
 namespace {
 
-constexpr int kConsumerWarps = 8;                     // warps that compute
-constexpr int kConsumers = kConsumerWarps * 32;        // 256 consumer threads
-constexpr int kThreads = kConsumers + 32;              // + one producer warp issuing the bulk copies
-constexpr int kWarps = kThreads / 32;
+constexpr int kConsumerWarps = 8;                // warps that compute
+constexpr int kConsumers = kConsumerWarps * 32;  // 256 consumer threads
+constexpr int kThreads = kConsumers + 32;        // + one producer warp issuing the tile loads
+constexpr int kPartCols = 32;                    // most basis columns a consumer lane holds in registers
 constexpr int kMaxStages = 8;
-constexpr int kMaxChunk = 256;                         // rows per chunk (tile box limit)
-constexpr size_t kStageTarget = 64 * 1024;            // bytes of one pipeline stage (target)
-constexpr size_t kStageBudget = 196 * 1024;           // bytes of all stages together
-// FP32 basis: two CTAs per SM (twice the consumer warps for the same bytes), each with about half
-// the stage budget; chunks of 128 rows (512-byte runs per column) whenever two stages fit, which
-// measured well ahead of 64 rows with more stages
-constexpr size_t kStageBudget32 = 100 * 1024;
-template <typename TS>
-constexpr int ctas_per_sm() { return sizeof(TS) == sizeof(float) ? 2 : 1; }
+constexpr size_t kStageBudget = 192 * 1024;      // bytes of all stages together
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -71,17 +55,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-// Bounded wait: returns false if the phase did not complete within kSpinLimit polls.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity) {
-  for (long long it = 0; it < kSpinLimit; ++it)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
+// Bounded wait: after kSpinLimit polls, or once another wait of the CTA has given up, it sets *gave_up
+// and returns; the caller goes on (every thread keeps meeting the CTA's barriers) and the column ends
+// with an error.
+__device__ __forceinline__ void mbar_wait_bounded(uint64_t *bar, uint32_t parity, volatile int *gave_up) {
+  if (mbar_try_wait(bar, parity)) return;
+  for (long long it = 0; it < kSpinLimit && !*gave_up; ++it)
+    if (mbar_try_wait(bar, parity)) return;
+  *gave_up = 1;
 }
 // 2-D tile load through a tensor map: box at (x = first row, y = first column).
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *tmap, int x, int y, uint64_t *bar) {
@@ -94,25 +75,9 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *tmap, 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Barrier 1 over the consumer warps only (the producer warp never joins it), with an OR-vote:
-// true on every consumer thread if any passed true.
-__device__ __forceinline__ bool consumer_sync_or(bool v) {
-  uint32_t out;
-  asm volatile(
-      "{\n"
-      " .reg .pred pi, po;\n"
-      " setp.ne.u32 pi, %1, 0;\n"
-      " bar.red.or.pred po, 1, %2, pi;\n"
-      " selp.u32 %0, 1, 0, po;\n"
-      "}\n"
-      : "=r"(out)
-      : "r"((uint32_t)v), "n"(kConsumers)
-      : "memory");
-  return out != 0;
-}
-// Barrier 1 over the consumer warps only, without a vote.
-__device__ __forceinline__ void consumer_sync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
+// Barrier `id` over `threads` threads of the CTA (the warps that share a group of rows).
+__device__ __forceinline__ void group_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
@@ -122,576 +87,470 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-struct PassParams {
+// Lane l < CPW returns the sum over the lanes of acc[l]: a halving exchange, 31 shuffles for 32 columns
+// where a tree per column takes 160.
+template <int CPW>
+__device__ __forceinline__ double lane_column_sums(const double (&acc)[CPW], int lane) {
+  double v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = i < CPW ? acc[i < CPW ? i : 0] : 0.0;
+#pragma unroll
+  for (int half = 16; half > 0; half >>= 1) {
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const bool up = (lane & half) != 0;
+      const double keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+    }
+  }
+  return v[0];
+}
+
+struct ColumnParams {
   GsPassArgs a;
   GsState *st;
-  double *coef;
   double *cnew;
-  double *partials;
-  int first;       // first pass of a column: action = DOT, coefficients start from zero
-  int plain_dot;   // plain BVDotVec: DOT only, no decision
-  int chunk;       // rows per chunk (power of two, 32..256)
-  int stages;      // pipeline stages (2..kMaxStages)
-  int box_cols;    // columns fetched by the 2-D tile load (jb, or jb+1 when w is column jb)
-  int stage_bytes; // bytes of one stage: CH rows of the jb basis columns (stored type) and of w (FP64)
+  double *partials;  // two buffers of G x (jb + 1) per-CTA dots, by parity of the pass
+  double eta;
+  double deftol;     // BV deftol = 10*PETSC_MACHINE_EPSILON (bvfunc.c:184)
+  int fresh;         // start of a run: the control block's counters and halt flag are replaced (not its error bits)
+  int plain_dot;     // plain BVDotVec: one DOT, no decision
+  int parts;         // warps that share a group of 32 rows (1, 2, 4, 8): each owns 1/parts of the columns
+  int stages;
   int nchunks;
-  int G;           // CTAs in the grid
 };
 
-// Shared scalars of the decision step.
-struct DecideShared {
-  int stage, pass, action, cont, lindep, err;
+// State of the DGKS machine of one column, kept by every CTA (all CTAs hold the same values).
+struct Decision {
+  int stage, pass, action, lindep, err;
   double onrm, nrm, scale;
-  double red[kWarps];
 };
 
-// BVOrthogonalizeGS's "finish a pass" logic (bvorthog.c:176-187, 209-214), run by thread 0.
-__device__ void finish_pass(DecideShared &d, const PassParams &p, double onrm, double nrm, bool have_next) {
-  const GsState *st = p.st;
-  const GsPassArgs &a = p.a;
-  // fast32: the first pass ran in FP32 arithmetic, so the FP64 correction pass is always taken
-  const bool refine =
-      d.pass < 3 && nrm != 0.0 && (fabs(nrm) < st->eta * fabs(onrm) || (a.fast32 && d.pass == 1));
+// BVOrthogonalizeGS's "finish a pass" logic (bvorthog.c:176-187, 209-214).  Returns true if the dot
+// just reduced is already the dot of the next pass (have_next) and that pass is to be taken.
+__device__ bool finish_pass(Decision &d, const ColumnParams &p, double onrm, double nrm, bool have_next) {
+  const bool refine = d.pass < 3 && nrm != 0.0 && fabs(nrm) < p.eta * fabs(onrm);
   if (refine) {
-    if (have_next) {
-      // The dot just reduced is already the dot of the next pass.
-      d.stage = kStageDotOfPass;
-      d.cont = 1;
-    } else {
-      d.action = kActUpdate | kActDot;
-      d.stage = kStageDotOfPass;
-      d.cont = 0;
-    }
-    return;
+    d.stage = kStageDotOfPass;
+    if (!have_next) d.action = kActUpdate | kActDot;
+    return have_next;
   }
-  const int lindep = !(nrm != 0.0 && fabs(nrm) >= st->eta * fabs(onrm));
-  d.lindep = lindep;
+  d.lindep = !(nrm != 0.0 && fabs(nrm) >= p.eta * fabs(onrm));
   d.nrm = nrm;
-  d.scale = (a.normalize && nrm != 1.0 && nrm != 0.0) ? 1.0 / nrm : 1.0;
+  d.scale = (p.a.normalize && nrm != 1.0 && nrm != 0.0) ? 1.0 / nrm : 1.0;
   d.action = (have_next ? 0 : kActUpdate) | (d.scale != 1.0 ? kActScale : 0);
   d.stage = kStageDone;
-  d.cont = 0;
-  if (a.hacc) a.hacc[a.jb] = lindep ? 0.0 : nrm;  // BV_SetValue(bv,k,k,h,...)
-  if (a.T) {
-    a.T[a.step] = (a.jb > 0) ? a.hacc[a.jb - 1] : 0.0;
-    a.T[a.ldt + a.step] = lindep ? 0.0 : nrm;
+  return false;
+}
+
+// The decision after a DOT, run by one warp: cnew_s holds the reduced dots, coef_s gets the
+// coefficients of the next UPDATE, hsum the accumulated ones (BV_AddCoefficients).
+__device__ void decide(Decision &d, const ColumnParams &p, const double *cnew_s, double *coef_s, double *hsum,
+                       int lane) {
+  const int jb = p.a.jb;
+  const double self = cnew_s[jb];
+  if (d.stage == kStageExplicitNorm) {
+    // BV_NormVecOrColumn: the norm of the updated vector
+    if (!finish_pass(d, p, d.onrm, (self < 0.0) ? 0.0 : sqrt(self), true)) return;
+  }
+  double sum = 0.0;
+  for (int i = lane; i < jb; i += 32) {
+    const double c = cnew_s[i];
+    coef_s[i] = c;
+    hsum[i] = d.pass == 0 ? c : hsum[i] + c;
+    sum = fma(c, c, sum);
+  }
+  sum = warp_sum(sum);  // BV_SquareSum
+  d.pass += 1;
+  if (p.a.column && !(self > -p.deftol)) d.err |= kDevErrInnerProduct;  // BV_SafeSqrt
+  const double onrm = (self < 0.0) ? 0.0 : sqrt(self);
+  const double t = onrm * onrm - sum;  // estimate |v'| from |v| (bvorthog.c:124-127)
+  if (t > 0.0) {
+    finish_pass(d, p, onrm, sqrt(t), false);
+  } else {
+    d.onrm = onrm;
+    d.action = kActUpdate | kActDot;  // explicit norm of the updated vector next
+    d.stage = kStageExplicitNorm;
   }
 }
 
-// DGKS decision on the reduced dot (cnew_s), run by the whole last CTA.
-__device__ void decide(const PassParams &p, const double *cnew_s, DecideShared &d) {
-  const GsPassArgs &a = p.a;
-  GsState *st = p.st;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    d.stage = p.first ? kStageDotOfPass : st->stage;
-    d.pass = p.first ? 0 : st->pass;
-    d.onrm = st->onrm;
-    d.action = kActNone;
-    d.lindep = 0;
-    d.err = 0;
-    d.nrm = 0.0;
-    d.scale = 1.0;
+// Grid-wide barrier on one word: the CTAs' increments cancel in the low bits and flip the top bit once
+// all have arrived, so the word carries over between launches of any grid size.  Every CTA is resident
+// (cooperative launch).  Called by one thread per CTA between __syncthreads(); false after kSpinLimit
+// polls.
+__device__ __forceinline__ unsigned grid_arrive(unsigned *word, int G) {
+  __threadfence();
+  return atomicAdd(word, blockIdx.x == 0 ? 0x80000000u - (unsigned)(G - 1) : 1u);
+}
+__device__ __forceinline__ bool grid_wait(unsigned *word, unsigned arrived) {
+  for (long long it = 0; it < kSpinLimit; ++it) {
+    unsigned now;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(word) : "memory");
+    if ((now ^ arrived) & 0x80000000u) return true;
   }
-  __syncthreads();
-  bool fresh = p.first != 0;
-  for (int iter = 0; iter < 4; ++iter) {
-    if (d.stage == kStageDotOfPass) {
-      // Coefficients of this pass: applied by the next UPDATE and accumulated (BV_AddCoefficients).
-      double local = 0.0;
-      for (int i = tid; i < a.jb; i += kThreads) {
-        const double c = cnew_s[i];
-        p.coef[i] = c;
-        if (a.hacc) a.hacc[i] = fresh ? c : a.hacc[i] + c;
-        local = fma(c, c, local);
-      }
-      local = warp_sum(local);
-      if (lane == 0) d.red[warp] = local;
-      __syncthreads();
-      if (tid == 0) {
-        double sum = 0.0;
-        for (int w = 0; w < kWarps; ++w) sum += d.red[w];  // BV_SquareSum
-        d.pass += 1;
-        const double self = cnew_s[a.jb];
-        if (a.column && !(self > -st->deftol)) d.err |= kDevErrInnerProduct;  // BV_SafeSqrt
-        const double onrm = (self < 0.0) ? 0.0 : sqrt(self);
-        const double t = onrm * onrm - sum;  // estimate |v'| from |v| (bvorthog.c:124-127)
-        if (t > 0.0) {
-          finish_pass(d, p, onrm, sqrt(t), false);
-        } else {
-          d.onrm = onrm;
-          d.action = kActUpdate | kActDot;  // explicit norm of the updated vector next
-          d.stage = kStageExplicitNorm;
-          d.cont = 0;
-        }
-      }
-    } else if (d.stage == kStageExplicitNorm) {
-      if (tid == 0) {
-        const double self = cnew_s[a.jb];
-        finish_pass(d, p, d.onrm, (self < 0.0) ? 0.0 : sqrt(self), true);  // BV_NormVecOrColumn
-      }
-    } else {
-      if (tid == 0) d.cont = 0;
-    }
-    fresh = false;
-    __syncthreads();
-    if (!d.cont) break;
-    __syncthreads();
-  }
-  if (tid == 0) {
-    st->action = d.action;
-    st->stage = d.stage;
-    st->pass = d.pass;
-    st->onrm = d.onrm;
-    st->err |= d.err;
-    if (d.stage == kStageDone) {
-      st->nrm = d.nrm;
-      st->scale = d.scale;
-      st->beta_out = d.nrm;
-      st->lindep = d.lindep;
-      if (d.lindep && a.step >= 0) {
-        st->halt = 1;
-        st->halt_step = a.step;
-      }
-    } else {
-      st->scale = 1.0;
-    }
-  }
+  return false;
 }
 
-// MAXCPW: largest number of dot columns one consumer warp owns (columns warp, warp+8, ...).
-//
-// Warp roles: warps 0..7 consume (update, scale, dot), warp 8 produces.  The
-// producer streams row chunks (w and the jb basis columns, one bulk copy per
-// column) into `stages` shared-memory stages; full[s] completes when a
-// stage's bytes have landed, empty[s] when the 8 consumer warps are done with
-// it.  Consumers synchronise among themselves only between the update (which
-// rewrites w) and the dot (which reads the new w).
-//
-// TS is the stored type of the basis: double, or float for the FP32 basis of the mixed-precision
-// solver (w, the coefficients and every product and sum stay FP64).
-template <int MAXCPW, typename TS>
-__global__ void __launch_bounds__(kThreads, ctas_per_sm<TS>()) gs_pass_kernel(PassParams p,
-                                                                             const __grid_constant__ CUtensorMap tmap) {
+// One column.  Warps 0..7 consume, warp 8 produces.  The producer streams row chunks of the jb basis
+// columns (one 2-D TMA tile load each) into a ring of shared-memory stages; full[s] completes when a
+// tile has landed, empty[s] when the consumer warps have copied it into registers.  The chunk's rows
+// form groups of 32, one row per lane; `parts` warps share a group, each holding its share of the
+// columns (CPW, jb / parts rounded up to the instantiated sizes: fixed trip counts, the columns past jb
+// are zeros that no load writes) of its lane's row in registers from the update to the dot, so a tile is
+// read from shared memory once, the update needs no exchange for jb <= 32 (parts = 1) and otherwise one
+// partial sum per warp and row behind a barrier of the group's warps alone, and the dots stay
+// lane-private across all chunks.  What bounds it: HBM for large n (8 n (jb + 1) bytes per pass), the
+// passes' latency for small n.
+//   * Passes alternate direction over the chunks, so a pass finds in L2 what the one before read last.
+//   * The pass that follows a DOT needs V again whatever is decided (unless the DOT was for an explicit
+//     norm), so its first tiles are loaded while the grid barrier, the reduction and the decision run.
+//   * w is read and written with plain loads and stores by the CTA that owns its rows (one chunk ahead);
+//     only V, which the kernel does not write, goes through the async proxy.
+// Measured (whole b200_bv_orthonormalize_column calls, refined columns, against five launches of a pass
+// kernel that read each tile twice and shared a row among all eight warps): n = 2,097,152 j = 8 198 ->
+// 144 us, j = 40 434 -> 359, j = 60 555 -> 523 (5.9 TB/s), j = 79 761 -> 658 (6.2 TB/s); n = 262,144
+// j = 60 135 -> 106; n = 10,000 j = 20 62 -> 55.  Alternating direction is worth 10% at n = 262,144
+// j = 60 and nothing at n = 2,097,152.  Trip counts taken from jb at run time instead of CPW: 636 us at
+// j = 60 (588 instructions per warp and tile, 150 so).
+template <int CPW>
+__global__ void __launch_bounds__(kThreads, 1) gs_column_kernel(ColumnParams p, const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages];
+  __shared__ __align__(16) double coef_s[kConsumerWarps * CPW];  // zero past jb
+  __shared__ double cnew_s[kMaxCols + 1], hsum[kMaxCols + 1];
+  __shared__ double red[kConsumerWarps][kMaxCols + 1];
+  __shared__ double upd[2][kConsumerWarps][32];  // partial update sums, by parity of the chunk
+  __shared__ Decision dsh;
+  __shared__ volatile int gave_up;
+  __shared__ int grid_ok;
   // Launched as a programmatic dependent of the previous kernel in the stream: wait until that
-  // grid has finished and its writes (the control block, coefficients, w) are visible, then let
-  // the next pass be launched at once (its CTAs take each SM as this grid's CTA leaves it).
+  // grid has finished and its writes (the control block, w) are visible, then let the next kernel
+  // be launched at once (its CTAs take each SM as this grid's CTA leaves it).
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" :::);
-  GsState *st = p.st;
   const GsPassArgs &a = p.a;
-  if (a.step >= 0 && st->halt && st->halt_step < a.step) return;
-  const int action = (p.first || p.plain_dot) ? (int)kActDot : st->action;
-  if (action == kActNone) return;
+  GsState *st = p.st;
+  if (a.step >= 0 && !p.fresh && st->halt && st->halt_step < a.step) return;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool producer = (warp == kConsumerWarps);
-  const int CH = p.chunk;
-  const int S = p.stages;
-  const int jb = a.jb;
-  const bool do_update = (action & kActUpdate) != 0;
-  const bool do_dot = (action & kActDot) != 0;
-  const bool do_scale = (action & kActScale) != 0;
-  const int ncl = (do_update || do_dot) ? jb : 0;  // basis columns streamed
-  const double scale = do_scale ? st->scale : 1.0;
-  // FP32 basis with fast32: the dot of the first pass and the update that applies its coefficients
-  // run in FP32 arithmetic (products and sums), the correction pass in FP64
-  const int passno = p.first ? 0 : st->pass;
-  const bool fast_dot = sizeof(TS) == sizeof(float) && a.fast32 && p.first && do_dot;
-  const bool fast_update = sizeof(TS) == sizeof(float) && a.fast32 && do_update && passno == 1;
-
-  // shared memory carve-up
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw);
-  uint64_t *empty = full + kMaxStages;
-  double *coef_s = reinterpret_cast<double *>(smem_raw + 128);
-  double *cacc = coef_s + kMaxCols;           // [kMaxCols + 1]
-  DecideShared *dsh = reinterpret_cast<DecideShared *>(cacc + kMaxCols + 1);
-  __shared__ int is_last, timed_out, n_issued;
-  __shared__ double upd[2 * kConsumers];      // partial update sums (TPR*CH = kConsumers per chunk), by chunk parity
-  __shared__ double wps[kMaxChunk];           // w' of the current chunk (updated and scaled), read by the dot
-  __shared__ float coef32_s[sizeof(TS) == sizeof(float) ? kMaxCols : 1];  // FP32 coefficients (fast update)
-  const size_t head = 128 + sizeof(double) * (2 * kMaxCols + 1) + ((sizeof(DecideShared) + 127) / 128) * 128;
-  unsigned char *stage_base = smem_raw + ((head + 127) / 128) * 128;
-  const size_t stage_bytes = (size_t)p.stage_bytes;
-  const size_t w_offset = (size_t)CH * jb * sizeof(TS);  // w follows the basis columns in a stage
-
+  const bool producer = warp == kConsumerWarps;
+  const int G = gridDim.x, S = p.stages, jb = a.jb, parts = p.parts;
+  const int CH = kConsumers / parts;
+  const uint32_t tile_bytes = (uint32_t)CH * (uint32_t)jb * 8u;                          // what a load brings
+  const uint32_t stage_bytes = (uint32_t)CH * (uint32_t)(parts * CPW) * 8u;  // with the zero columns past jb
+  unsigned char *stage_base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], kConsumerWarps);
     }
     fence_mbar_init();
-    timed_out = 0;
-    n_issued = 0;
+    gave_up = 0;
+    dsh = Decision{kStageDotOfPass, 0, kActDot, 0, 0, 0.0, 0.0, 1.0};
   }
-  for (int i = tid; i < jb; i += kThreads) coef_s[i] = do_update ? p.coef[i] : 0.0;
-  if constexpr (sizeof(TS) == sizeof(float))
-    if (fast_update)
-      for (int i = tid; i < jb; i += kThreads) coef32_s[i] = __double2float_rn(p.coef[i]);
+  for (int i = tid; i < kConsumerWarps * CPW; i += kThreads) coef_s[i] = 0.0;
+  for (int s = 0; s < S; ++s) {
+    double *pad = reinterpret_cast<double *>(stage_base + (size_t)s * stage_bytes) + (size_t)CH * jb;
+    for (int i = tid; i < CH * (parts * CPW - jb); i += kThreads) pad[i] = 0.0;
+  }
   __syncthreads();
 
-  const int G = p.G;
   const int nmine = (p.nchunks > (int)blockIdx.x) ? (p.nchunks - 1 - (int)blockIdx.x) / G + 1 : 0;
-  double *Vw = a.wvec ? a.wvec : a.V + (size_t)a.wcol * a.ld;
-  int consumed = 0;
+  double *Vw = a.V + (size_t)a.wcol * a.ld;
+  // this warp's group of rows and share of the columns
+  const int group = warp / parts, part = warp % parts;
+  const int c0 = part * CPW;
+  const int ldp = jb + 1;
 
-  // dot accumulators: lane-private partial sums of the columns this warp owns, across all chunks
-  double acc[MAXCPW];
-#pragma unroll
-  for (int t = 0; t < MAXCPW; ++t) acc[t] = 0.0;
-
-  if (producer) {
-    for (int i = 0; i < nmine; ++i) {
-      const int s = i % S;
-      if (i >= S) {
-        const bool ok = mbar_wait_bounded(&empty[s], (uint32_t)(((i / S) - 1) & 1));
-        if (!__all_sync(0xffffffffu, ok)) {
-          if (lane == 0) timed_out = 1;
-          break;
+  int tile = 0;        // tiles issued (producer) or consumed (consumers) so far
+  int ahead = 0;       // producer: tiles of the coming pass that are already issued
+  unsigned npass = 0;
+  unsigned long long bytes = 0;
+  bool ok = true;
+  for (int pass = 0;; ++pass) {
+    const int action = dsh.action;
+    const bool do_update = (action & kActUpdate) != 0, do_dot = (action & kActDot) != 0;
+    const bool do_scale = (action & kActScale) != 0;
+    const bool rewrite = do_update || do_scale;
+    const bool tiles = (do_update || do_dot) && jb > 0;
+    const bool next_tiles = tiles && do_dot && dsh.stage == kStageDotOfPass && !p.plain_dot;
+    const double scale = do_scale ? dsh.scale : 1.0;
+    // chunk i of the pass, in the pass's direction
+    auto chunk_row = [&](int i, int ps) {
+      const int k = (ps & 1) ? nmine - 1 - i : i;
+      return ((long long)blockIdx.x + (long long)k * G) * CH;
+    };
+    if (producer) {
+      if (lane == 0 && tiles) {
+        const int total = nmine + (next_tiles ? min(S, nmine) : 0);
+        for (int i = ahead; i < total; ++i, ++tile) {
+          const int s = tile % S;
+          if (tile >= S) mbar_wait_bounded(&empty[s], (uint32_t)(((tile / S) - 1) & 1), &gave_up);
+          if (gave_up) break;
+          const bool next = i >= nmine;
+          mbar_arrive_expect_tx(&full[s], tile_bytes);
+          tma_load_2d(stage_base + (size_t)s * stage_bytes, &tmap, (int)chunk_row(next ? i - nmine : i, pass + (next ? 1 : 0)),
+                      0, &full[s]);
         }
-      }
-      const long long r0 = ((long long)blockIdx.x + (long long)i * G) * CH;
-      const int rows = (int)min((long long)CH, (long long)a.n - r0);
-      unsigned char *buf = stage_base + (size_t)s * stage_bytes;
-      if (lane == 0) {
-        // one tile load brings the basis columns (and w when it is column jb); rows past n read as zeros
-        const bool tile = ncl > 0;
-        const bool w_in_tile = tile && p.box_cols == jb + 1;
-        const uint32_t wbytes = w_in_tile ? 0u : (uint32_t)(((rows * 8) + 15) & ~15);
-        const uint32_t tbytes = tile ? (uint32_t)CH * (uint32_t)sizeof(TS) * (uint32_t)p.box_cols : 0u;
-        mbar_arrive_expect_tx(&full[s], tbytes + wbytes);
-        if (tile) tma_load_2d(buf, &tmap, (int)r0, 0, &full[s]);
-        if (!w_in_tile) bulk_load(buf + w_offset, Vw + r0, wbytes, &full[s]);
-        n_issued = i + 1;
+        ahead = total - nmine;
       }
       __syncwarp();
-    }
-  } else {
-    // Update mapping: the chunk's rows form CH/32 groups of 32; the 8 consumer warps split into
-    // TPR = 8/(CH/32) parts, warp w taking row group w % (CH/32) and columns part, part+TPR, ...
-    // (one column, 32 consecutive rows per instruction: no bank conflicts).  Partial sums meet
-    // in upd[part][row] behind the chunk's barrier; consumer thread r then folds them into row r
-    // of w' (fixed order), keeps it in wps for the dot and writes it back to global memory, and
-    // a second barrier hands wps to the dot.
-    const int groups = CH / 32;  // 1..8
-    const int TPR = kConsumerWarps / groups;
-    const int part = warp / groups;
-    const int urow = (warp % groups) * 32 + lane;
-    for (int i = 0; i < nmine; ++i) {
-      const int s = i % S;
-      const bool ok = mbar_wait_bounded(&full[s], (uint32_t)((i / S) & 1));
-      const long long r0 = ((long long)blockIdx.x + (long long)i * G) * CH;
-      const int rows = (int)min((long long)CH, (long long)a.n - r0);
-      const unsigned char *sbuf = stage_base + (size_t)s * stage_bytes;
-      const TS *Vs = reinterpret_cast<const TS *>(sbuf);  // column c at Vs + c*CH, w after the basis
-      const double *wsrc = reinterpret_cast<const double *>(sbuf + w_offset);
-      double *up = upd + (i & 1) * kConsumers;  // partial update sums of this chunk
-      const bool rewrite = do_update || do_scale;
-      if (rewrite) {
-        if (ok && do_update) {
-          if constexpr (sizeof(TS) == sizeof(double)) {
-            double s0 = 0.0, s1 = 0.0;
-            int c = part;
-            for (; c + TPR < jb; c += 2 * TPR) {
-              s0 = fma(Vs[(size_t)c * CH + urow], coef_s[c], s0);
-              s1 = fma(Vs[(size_t)(c + TPR) * CH + urow], coef_s[c + TPR], s1);
-            }
-            if (c < jb) s0 = fma(Vs[(size_t)c * CH + urow], coef_s[c], s0);
-            up[part * CH + urow] = s0 + s1;
-          } else if (fast_update) {
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-            int c = part;
-            for (; c + 3 * TPR < jb; c += 4 * TPR) {
-              s0 = fmaf((float)Vs[(size_t)c * CH + urow], coef32_s[c], s0);
-              s1 = fmaf((float)Vs[(size_t)(c + TPR) * CH + urow], coef32_s[c + TPR], s1);
-              s2 = fmaf((float)Vs[(size_t)(c + 2 * TPR) * CH + urow], coef32_s[c + 2 * TPR], s2);
-              s3 = fmaf((float)Vs[(size_t)(c + 3 * TPR) * CH + urow], coef32_s[c + 3 * TPR], s3);
-            }
-            for (; c < jb; c += TPR) s0 = fmaf((float)Vs[(size_t)c * CH + urow], coef32_s[c], s0);
-            up[part * CH + urow] = (double)((s0 + s1) + (s2 + s3));
-          } else {
-            // four independent chains: the FP32 basis doubles the columns a chunk holds per byte
+    } else {
+      double acc[CPW], self = 0.0;
+#pragma unroll
+      for (int t = 0; t < CPW; ++t) acc[t] = 0.0;
+      const int lrow = group * 32 + lane;
+      auto load_w = [&](int i) {
+        const long long row = chunk_row(i, pass) + lrow;
+        return (i < nmine && row < a.n) ? __ldcg(Vw + row) : 0.0;
+      };
+      double wnext = load_w(0);
+      for (int i = 0; i < nmine; ++i) {
+        const long long row = chunk_row(i, pass) + lrow;
+        double wv = wnext;
+        wnext = load_w(i + 1);
+        double v[CPW];
+        if (tiles) {
+          const int s = tile % S;
+          mbar_wait_bounded(&full[s], (uint32_t)((tile / S) & 1), &gave_up);
+          const double *Vs = reinterpret_cast<const double *>(stage_base + (size_t)s * stage_bytes) + (size_t)c0 * CH + lrow;
+#pragma unroll
+          for (int t = 0; t < CPW; ++t) v[t] = Vs[t * CH];
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty[s]);  // copied out: the next tile load may overwrite it
+          ++tile;
+        }
+        if (do_update) {
+          double tot = 0.0;
+          if (tiles) {
             double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-            int c = part;
-            for (; c + 3 * TPR < jb; c += 4 * TPR) {
-              s0 = fma((double)Vs[(size_t)c * CH + urow], coef_s[c], s0);
-              s1 = fma((double)Vs[(size_t)(c + TPR) * CH + urow], coef_s[c + TPR], s1);
-              s2 = fma((double)Vs[(size_t)(c + 2 * TPR) * CH + urow], coef_s[c + 2 * TPR], s2);
-              s3 = fma((double)Vs[(size_t)(c + 3 * TPR) * CH + urow], coef_s[c + 3 * TPR], s3);
+            const double2 *cf = reinterpret_cast<const double2 *>(coef_s + c0);
+#pragma unroll
+            for (int t = 0; t < CPW; t += 4) {
+              const double2 ca = cf[t / 2], cb = cf[t / 2 + 1];
+              s0 = fma(v[t], ca.x, s0);
+              s1 = fma(v[t + 1], ca.y, s1);
+              s2 = fma(v[t + 2], cb.x, s2);
+              s3 = fma(v[t + 3], cb.y, s3);
             }
-            for (; c < jb; c += TPR) s0 = fma((double)Vs[(size_t)c * CH + urow], coef_s[c], s0);
-            up[part * CH + urow] = (s0 + s1) + (s2 + s3);
+            tot = (s0 + s1) + (s2 + s3);
           }
+          if (parts > 1) {
+            double(*up)[32] = upd[i & 1];
+            up[warp][lane] = tot;
+            group_sync(1 + group, parts * 32);
+            tot = 0.0;
+            for (int r = 0; r < parts; ++r) tot += up[group * parts + r][lane];  // the same order in every warp
+          }
+          wv -= tot;
         }
-        if (consumer_sync_or(!ok)) break;  // partial sums complete (and a timed-out wait is agreed on)
-      } else if (!ok) {
-        break;
-      }
-      // w' = w - sum of the parts (fixed order), scaled: once per row, for the dot and global memory
-      if (rewrite) {
-        for (int r = tid; r < rows; r += kConsumers) {
-          double wv = wsrc[r];
-          if (do_update) {
-            double tot = 0.0;
-            for (int q = 0; q < TPR; ++q) tot += up[q * CH + r];
-            wv -= tot;
-          }
+        if (rewrite) {
           if (do_scale) wv *= scale;
-          wps[r] = wv;
-          Vw[r0 + r] = wv;
+          if (part == 0 && row < a.n) Vw[row] = wv;
         }
-        if (do_dot) consumer_sync();
-      }
-      const double *wd = rewrite ? wps : wsrc;  // the vector the dot multiplies
-      if (do_dot && fast_dot) {
-        // FP32 products summed in FP32 over the chunk's rows of this lane, then added in FP64
-        float facc[MAXCPW];
+        if (do_dot) {
+          if (tiles) {
 #pragma unroll
-        for (int t = 0; t < MAXCPW; ++t) facc[t] = 0.f;
-        for (int r = lane; r < rows; r += 32) {
-          const float wr = __double2float_rn(wd[r]);
-#pragma unroll
-          for (int t = 0; t < MAXCPW; ++t) {
-            const int c = warp + kConsumerWarps * t;
-            if (c < jb) facc[t] = fmaf((float)Vs[(size_t)c * CH + r], wr, facc[t]);
-            else if (c == jb) facc[t] = fmaf(wr, wr, facc[t]);
+            for (int t = 0; t < CPW; ++t) acc[t] = fma(v[t], wv, acc[t]);
           }
-        }
-#pragma unroll
-        for (int t = 0; t < MAXCPW; ++t) acc[t] += (double)facc[t];
-      } else if (do_dot) {
-        for (int r = lane; r < rows; r += 32) {
-          const double wr = wd[r];
-#pragma unroll
-          for (int t = 0; t < MAXCPW; ++t) {
-            const int c = warp + kConsumerWarps * t;
-            if (c < jb) acc[t] = fma((double)Vs[(size_t)c * CH + r], wr, acc[t]);
-            else if (c == jb) acc[t] = fma(wr, wr, acc[t]);
-          }
+          if (part == 0) self = fma(wv, wv, self);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);  // stage only read here: the next bulk copy may overwrite it
-      consumed = i + 1;
+      if (do_dot) {
+        const double mine = lane_column_sums(acc, lane);
+        if (lane < CPW && c0 + lane < jb) red[group][c0 + lane] = mine;
+        self = warp_sum(self);
+        if (part == 0 && lane == 0) red[group][jb] = self;
+      }
     }
-    if (lane == 0 && consumed < nmine) timed_out = 1;
-  }
-  __syncthreads();
-  if (timed_out) {
-    // Drain the copies still in flight (bounded), report, and leave.
-    if (tid == 0) {
-      atomicOr(&st->err, (int)kDevErrTimeout);
-      for (int i = consumed; i < n_issued; ++i) (void)mbar_wait_bounded(&full[i % S], (uint32_t)((i / S) & 1));
+    ++npass;
+    // algorithmic traffic of this pass: streamed columns + w read, w written back if changed
+    bytes += (unsigned long long)a.n * 8ull * ((tiles ? jb : 0) + 1 + (rewrite ? 1 : 0));
+    if (!do_dot) break;
+    __syncthreads();
+    double *pb = p.partials + (size_t)(pass & 1) * G * ldp;
+    const int groups = kConsumerWarps / parts;
+    for (int c = tid; c <= jb; c += kThreads) {
+      double sacc = 0.0;
+      for (int g = 0; g < groups; ++g) sacc += red[g][c];
+      __stcg(pb + (size_t)blockIdx.x * ldp + c, sacc);
     }
     __syncthreads();
-    return;
-  }
-
-  // per-CTA column sums -> partials[c * G + cta]
-  if (do_dot && !producer) {
-#pragma unroll
-    for (int t = 0; t < MAXCPW; ++t) {
-      const int c = warp + kConsumerWarps * t;
-      const double v = warp_sum(acc[t]);
-      if (lane == 0 && c <= jb) p.partials[(size_t)c * G + blockIdx.x] = v;
-    }
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) is_last = (atomicAdd(&st->ticket, 1u) == (unsigned)(G - 1));
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  if (tid == 0) {
-    // algorithmic traffic of this pass: streamed columns + w read, w written back if changed
-    st->bytes += (unsigned long long)a.n *
-                 ((unsigned long long)sizeof(TS) * ncl + 8ull * (1ull + ((do_update || do_scale) ? 1ull : 0ull)));
-    st->passes += 1;
-  }
-  if (!do_dot) {
-    // The final UPDATE/SCALE of a column is done: later follow-up launches idle.
     if (tid == 0) {
-      st->ticket = 0u;
-      st->action = kActNone;
+      const unsigned arrived = grid_arrive(&st->ticket, G);
+      // a plain dot is reduced by CTA 0 alone
+      grid_ok = (p.plain_dot && blockIdx.x != 0) || grid_wait(&st->ticket, arrived);
+      __threadfence();
     }
-    return;
+    __syncthreads();
+    ok = grid_ok != 0;
+    if (!ok || (p.plain_dot && blockIdx.x != 0)) break;
+    // Fixed-order sum over the CTAs: warp w adds CTAs w, w + 8, ... with one column per lane (32
+    // independent coalesced loads in flight per warp and column group), then the warps in order.
+    if (!producer) {
+      for (int c = lane; c <= jb; c += 32) {
+        double sacc = 0.0;
+#pragma unroll 8
+        for (int b = warp; b < G; b += kConsumerWarps) sacc += __ldcg(pb + (size_t)b * ldp + c);
+        red[warp][c] = sacc;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      for (int c = lane; c <= jb; c += 32) {
+        double sacc = 0.0;
+#pragma unroll
+        for (int w = 0; w < kConsumerWarps; ++w) sacc += red[w][c];
+        cnew_s[c] = sacc;
+      }
+      __syncwarp();
+      if (!p.plain_dot) {
+        Decision d = dsh;
+        decide(d, p, cnew_s, coef_s, hsum, lane);
+        __syncwarp();
+        if (lane == 0) dsh = d;
+      }
+    }
+    __syncthreads();
+    if (p.plain_dot || dsh.action == kActNone || gave_up) break;
   }
 
-  // Fixed-order reduction across CTAs: lane b sums CTAs b, b+32, ...; then a fixed shuffle tree.
-  double *cnew_s = cacc;
-  for (int c = warp; c <= jb; c += kWarps) {
-    double sacc = 0.0;
-    for (int b = lane; b < G; b += 32) sacc += __ldcg(p.partials + (size_t)c * G + b);
-    sacc = warp_sum(sacc);
-    if (lane == 0) {
-      cnew_s[c] = sacc;
-      p.cnew[c] = sacc;
-    }
-  }
   __syncthreads();
-  if (tid == 0) st->ticket = 0u;
-  if (p.plain_dot) return;
-  decide(p, cnew_s, *dsh);
-}
-
-// bytes of one pipeline stage: CH rows of jb basis columns of ts bytes each, then CH rows of w (FP64)
-size_t pass_stage_bytes(int jb, int CH, size_t ts) { return (size_t)CH * ((size_t)jb * ts + sizeof(double)); }
-
-size_t pass_smem_bytes(int jb, int CH, int stages, size_t ts) {
-  const size_t head = 128 + sizeof(double) * (2 * kMaxCols + 1) + ((sizeof(DecideShared) + 127) / 128) * 128;
-  return ((head + 127) / 128) * 128 + (size_t)stages * pass_stage_bytes(jb, CH, ts);
-}
-
-// Rows per chunk: the largest power of two (32..256, the tile box limit) whose stage fits the target size.
-int pass_chunk_rows(int jb, size_t ts) {
-  if (ts == sizeof(float)) {
-    int ch = kMaxChunk / 2;
-    while (ch > 32 && 2 * pass_stage_bytes(jb, ch, ts) > kStageBudget32) ch /= 2;
-    return ch;
+  if (blockIdx.x == 0) {
+    if (p.plain_dot) {
+      if (ok)
+        for (int c = tid; c <= jb; c += kThreads) p.cnew[c] = cnew_s[c];
+    } else if (ok && dsh.stage == kStageDone) {
+      const Decision &d = dsh;
+      if (a.hacc) {
+        for (int c = tid; c < jb; c += kThreads) a.hacc[c] = hsum[c];
+        if (tid == 0) a.hacc[jb] = d.lindep ? 0.0 : d.nrm;  // BV_SetValue(bv,k,k,h,...)
+      }
+      if (tid == 0) {
+        if (a.T) {
+          a.T[a.step] = jb > 0 ? hsum[jb - 1] : 0.0;
+          a.T[a.ldt + a.step] = d.lindep ? 0.0 : d.nrm;
+        }
+        st->beta_out = d.nrm;
+        st->lindep = d.lindep;
+        st->halt = d.lindep && a.step >= 0;
+        st->halt_step = a.step;
+      }
+    }
+    if (tid == 0) {
+      if (dsh.err) atomicOr(&st->err, dsh.err);
+      st->bytes = (p.fresh ? 0 : st->bytes) + bytes;
+      st->passes = (p.fresh ? 0 : st->passes) + (int)npass;
+    }
   }
-  const size_t rows = kStageTarget / ((size_t)jb * ts + sizeof(double));
-  int ch = 32;
-  while (ch < kMaxChunk && (size_t)(2 * ch) <= rows) ch *= 2;
-  return ch;
+  if (!ok || gave_up) {
+    // report, and let the copies still in flight land (bounded) before the CTA leaves
+    if (tid == 0) atomicOr(&st->err, (int)kDevErrTimeout);
+    if (producer && lane == 0)
+      for (int t = tile > S ? tile - S : 0; t < tile; ++t)
+        for (long long it = 0; it < kSpinLimit && !mbar_try_wait(&full[t % S], (uint32_t)((t / S) & 1)); ++it) {
+        }
+  }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     void *ptr = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
-  }
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      ptr = nullptr;
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
+  }();
   return fn;
 }
 
-// Tensor map over the basis: dim 0 = rows (n, contiguous), dim 1 = columns (stride ld), box CH x box_cols.
-cudaError_t make_tmap(CUtensorMap *tm, const GsPassArgs &a, int CH, int box_cols, int total_cols) {
-  const bool f32 = a.V32 != nullptr;
+// Tensor map over the basis: dim 0 = rows (n, contiguous), dim 1 = columns (stride ld), box rows x cols.
+cudaError_t make_tmap(CUtensorMap *tm, const GsPassArgs &a, int rows, int cols) {
   memset(tm, 0, sizeof(*tm));
-  if (box_cols <= 0) return cudaSuccess;  // no tile load in this pass
+  if (cols <= 0) return cudaSuccess;  // no tile load in this column
   PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
-  const cuuint64_t dims[2] = {(cuuint64_t)a.n, (cuuint64_t)total_cols};
-  const cuuint64_t strides[1] = {f32 ? (cuuint64_t)a.ld32 * sizeof(float) : (cuuint64_t)a.ld * sizeof(double)};
-  const cuuint32_t box[2] = {(cuuint32_t)CH, (cuuint32_t)box_cols};
+  const cuuint64_t dims[2] = {(cuuint64_t)a.n, (cuuint64_t)a.total_cols};
+  const cuuint64_t strides[1] = {(cuuint64_t)a.ld * sizeof(double)};
+  const cuuint32_t box[2] = {(cuuint32_t)rows, (cuuint32_t)cols};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(tm, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2,
-                   f32 ? (void *)a.V32 : (void *)a.V, dims, strides, box, estr,
+  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void *)a.V, dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-int pass_stages(int jb, int CH, size_t ts) {
-  const size_t stage = pass_stage_bytes(jb, CH, ts);
-  size_t s = (ts == sizeof(double) ? kStageBudget : kStageBudget32) / stage;
-  if (s > (size_t)kMaxStages) s = kMaxStages;
-  return (int)s;
+// Warps that share a group of rows: the fewest whose lanes can hold the columns (32 doubles of the row
+// and as many dots).  More warps with fewer columns each cost a barrier and smaller tiles: n = 2,097,152
+// j = 50 takes 424 us with 32 columns a lane, 564 with 24 or 16; j = 79 658, 659 and 1002.
+int column_parts(int jb) {
+  int parts = 1;
+  while (parts < kConsumerWarps && jb > parts * kPartCols) parts *= 2;
+  return parts;
 }
 
-template <int M, typename TS>
-cudaError_t launch_pass_t(const PassParams &p, const CUtensorMap &tm, size_t smem, cudaStream_t stream) {
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 64 && !attr_set[dev]) {
-    cudaError_t e = allow_max_dynamic_smem(gs_pass_kernel<M, TS>);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
-  }
+template <int CPW>
+cudaError_t launch_column_t(ColumnParams &p, int G, cudaStream_t stream) {
+  const GsPassArgs &a = p.a;
+  const int CH = kConsumers / p.parts;
+  const size_t stage = (size_t)CH * p.parts * CPW * sizeof(double);
+  p.stages = (int)(kStageBudget / stage);
+  if (p.stages > kMaxStages) p.stages = kMaxStages;
+  CUtensorMap tm;
+  cudaError_t e = make_tmap(&tm, a, CH, a.jb);
+  if (e != cudaSuccess) return e;
+  if ((e = allow_max_dynamic_smem(gs_column_kernel<CPW>)) != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)p.G);
+  cfg.gridDim = dim3((unsigned)G);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = stage * p.stages + 128;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeCooperative;  // the CTAs meet at grid barriers
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gs_pass_kernel<M, TS>, p, tm);
+  cfg.numAttrs = 2;
+  e = cudaLaunchKernelEx(&cfg, gs_column_kernel<CPW>, p, tm);
+  count_launch();
+  return e;
 }
 
-cudaError_t launch_pass(const GsPassArgs &a, const GsWork &w, int first, int plain_dot, cudaStream_t stream) {
-  PassParams p;
+cudaError_t launch_column(const GsPassArgs &a, const GsWork &w, double eta, int fresh, int plain_dot,
+                          cudaStream_t stream) {
+  if (a.jb < 0 || a.jb >= kMaxCols) return cudaErrorInvalidValue;
+  ColumnParams p;
   p.a = a;
   p.st = w.st;
-  p.coef = w.coef;
   p.cnew = w.cnew;
   p.partials = w.partials;
-  p.first = first;
+  p.eta = eta;
+  p.deftol = 10.0 * 2.220446049250313e-16;
+  p.fresh = fresh;
   p.plain_dot = plain_dot;
-  const bool f32 = a.V32 != nullptr;
-  const size_t ts = f32 ? sizeof(float) : sizeof(double);
-  if (f32 && !a.wvec) return cudaErrorInvalidValue;  // w is FP64 and kept apart from an FP32 basis
-  p.chunk = pass_chunk_rows(a.jb, ts);
-  p.stages = pass_stages(a.jb, p.chunk, ts);
-  p.stage_bytes = (int)pass_stage_bytes(a.jb, p.chunk, ts);
-  if (p.stages < 2) return cudaErrorInvalidValue;
-  p.nchunks = (a.n + p.chunk - 1) / p.chunk;
-  int G = w.num_sms * (f32 ? ctas_per_sm<float>() : 1);
-  if (G > w.max_ctas) G = w.max_ctas;
+  p.parts = column_parts(a.jb);
+  const int CH = kConsumers / p.parts;
+  p.nchunks = (a.n + CH - 1) / CH;
+  int G = w.num_sms < w.max_ctas ? w.num_sms : w.max_ctas;
   if (G > p.nchunks) G = p.nchunks;
-  if (G < 1) G = 1;
-  p.G = G;
-  const size_t smem = pass_smem_bytes(a.jb, p.chunk, p.stages, ts);
-  if (smem + 4096 > max_dynamic_smem()) return cudaErrorInvalidValue;
-  // w is column jb in the column variant: one box covers basis and w
-  p.box_cols = (a.wcol == a.jb && !a.wvec && !f32) ? a.jb + 1 : a.jb;
-  CUtensorMap tm;
-  cudaError_t e = make_tmap(&tm, a, p.chunk, p.box_cols, a.total_cols);
-  if (e != cudaSuccess) return e;
-  const int cpw = (a.jb + 1 + kConsumerWarps - 1) / kConsumerWarps;  // dot columns per consumer warp (basis + self)
-  if (f32) {
-    if (cpw <= 2) e = launch_pass_t<2, float>(p, tm, smem, stream);
-    else if (cpw <= 4) e = launch_pass_t<4, float>(p, tm, smem, stream);
-    else if (cpw <= 8) e = launch_pass_t<8, float>(p, tm, smem, stream);
-    else if (cpw <= 12) e = launch_pass_t<12, float>(p, tm, smem, stream);
-    else if (cpw <= 16) e = launch_pass_t<16, float>(p, tm, smem, stream);
-    else if (cpw <= 32) e = launch_pass_t<32, float>(p, tm, smem, stream);
-    else return cudaErrorInvalidValue;
-  } else if (cpw <= 2) e = launch_pass_t<2, double>(p, tm, smem, stream);
-  else if (cpw <= 4) e = launch_pass_t<4, double>(p, tm, smem, stream);
-  else if (cpw <= 8) e = launch_pass_t<8, double>(p, tm, smem, stream);
-  else if (cpw <= 12) e = launch_pass_t<12, double>(p, tm, smem, stream);
-  else if (cpw <= 16) e = launch_pass_t<16, double>(p, tm, smem, stream);
-  else if (cpw <= 32) e = launch_pass_t<32, double>(p, tm, smem, stream);
-  else return cudaErrorInvalidValue;
-  count_launch();
-  return e;
+  const int q = (a.jb + p.parts - 1) / p.parts;  // columns per warp
+  if (q <= 4) return launch_column_t<4>(p, G, stream);
+  if (q <= 8) return launch_column_t<8>(p, G, stream);
+  if (q <= 12) return launch_column_t<12>(p, G, stream);
+  if (q <= 16) return launch_column_t<16>(p, G, stream);
+  if (q <= 20) return launch_column_t<20>(p, G, stream);
+  if (q <= 24) return launch_column_t<24>(p, G, stream);
+  if (q <= 28) return launch_column_t<28>(p, G, stream);
+  return launch_column_t<32>(p, G, stream);
 }
 
-}  // namespace
-
-namespace {
-__global__ void gs_reset_kernel(GsState *st, double eta) {
+__global__ void gs_reset_kernel(GsState *st) {
   GsState h;
   memset(&h, 0, sizeof(h));
-  h.eta = eta;
-  h.deftol = 10.0 * 2.220446049250313e-16;  // BV deftol = 10*PETSC_MACHINE_EPSILON (bvfunc.c:184)
   h.halt_step = -1;
-  h.scale = 1.0;
   *st = h;
-}
-}  // namespace
-
-cudaError_t gs_state_reset(const GsWork &w, double eta, cudaStream_t stream) {
-  gs_reset_kernel<<<1, 1, 0, stream>>>(w.st, eta);
-  count_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t gs_orthogonalize_launch(const GsPassArgs &a, const GsWork &w, cudaStream_t stream) {
-  if (a.jb < 0 || a.jb >= kMaxCols) return cudaErrorInvalidValue;
-  cudaError_t e = launch_pass(a, w, 1, 0, stream);
-  // Worst case: three passes whose norm estimates all need the explicit norm,
-  // then a final scale: four follow-up launches (idle ones return at once).
-  for (int k = 0; k < 4 && e == cudaSuccess; ++k) e = launch_pass(a, w, 0, 0, stream);
-  return e;
 }
 
 // out[0] = the norm, out[1] = the lindep flag, out[2] = the device error bits of the last column
@@ -702,6 +561,19 @@ __global__ void gs_record_kernel(const GsState *__restrict__ st, double *out) {
   out[2] = (double)st->err;
 }
 
+}  // namespace
+
+cudaError_t gs_state_reset(const GsWork &w, cudaStream_t stream) {
+  gs_reset_kernel<<<1, 1, 0, stream>>>(w.st);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t gs_orthogonalize_launch(const GsPassArgs &a, const GsWork &w, double eta, bool fresh,
+                                    cudaStream_t stream) {
+  return launch_column(a, w, eta, fresh ? 1 : 0, 0, stream);
+}
+
 cudaError_t gs_record_launch(const GsWork &w, double *out, cudaStream_t stream) {
   gs_record_kernel<<<1, 1, 0, stream>>>(w.st, out);
   count_launch();
@@ -709,8 +581,7 @@ cudaError_t gs_record_launch(const GsWork &w, double *out, cudaStream_t stream) 
 }
 
 cudaError_t gs_dot_launch(const GsPassArgs &a, const GsWork &w, cudaStream_t stream) {
-  if (a.jb < 0 || a.jb >= kMaxCols) return cudaErrorInvalidValue;
-  return launch_pass(a, w, 0, 1, stream);
+  return launch_column(a, w, 0.0, 0, 1, stream);
 }
 
 }  // namespace b200

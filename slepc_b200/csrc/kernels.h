@@ -127,9 +127,8 @@ cudaError_t spmv_launch(int n, const int *rowptr, const int *colind, const doubl
 // Device workspace of one BV for the Gram-Schmidt kernels.
 struct GsWork {
   GsState *st;        // control block
-  double *coef;       // [kMaxCols] coefficients applied by the next UPDATE
-  double *cnew;       // [kMaxCols+1] result of the last reduced dot
-  double *partials;   // [(kMaxCols+1) * max_ctas] per-CTA partial dots
+  double *cnew;       // [kMaxCols+1] result of the last plain dot
+  double *partials;   // [2 * (kMaxCols+1) * max_ctas] per-CTA partial dots of two passes
   int max_ctas;
   int num_sms;
 };
@@ -146,22 +145,14 @@ struct GsPassArgs {
   int normalize;  // scale by 1/norm at the end
   int column;     // 1: column variant (BV_SafeSqrt check on w^T w)
   int total_cols; // columns allocated from V (bounds of the tile loads)
-  // FP32 basis (mixed-precision solver): when V32 is set the basis columns are read from V32
-  // (leading dimension ld32) and the vector being orthogonalised is the FP64 vector wvec (n + 2
-  // entries allocated); wvec may also be set with an FP64 basis.
-  const float *V32;
-  int ld32;
-  double *wvec;
-  // with V32: the first CGS pass (its dot and the update applying its coefficients) in FP32
-  // arithmetic, and the FP64 DGKS correction pass always taken
-  int fast32;
 };
 
-// Enqueue the full CGS + DGKS("if needed") orthogonalisation of one column:
-// a first dot pass plus the follow-up passes the device decides on.
-cudaError_t gs_orthogonalize_launch(const GsPassArgs &a, const GsWork &w, cudaStream_t stream);
-// Initialise the control block (eta, deftol, clears halt/err) -- once per run.
-cudaError_t gs_state_reset(const GsWork &w, double eta, cudaStream_t stream);
+// Enqueue the full CGS + DGKS("if needed") orthogonalisation of one column with threshold eta (one
+// cooperative launch).  fresh: the column starts a run (or stands alone), so the control block's
+// counters and halt flag start from it.
+cudaError_t gs_orthogonalize_launch(const GsPassArgs &a, const GsWork &w, double eta, bool fresh, cudaStream_t stream);
+// Clear the control block (at creation, and after an error has been read back).
+cudaError_t gs_state_reset(const GsWork &w, cudaStream_t stream);
 // out[0..2] = norm, lindep flag and error bits of the last orthogonalisation (no host sync).
 cudaError_t gs_record_launch(const GsWork &w, double *out, cudaStream_t stream);
 // Plain dots q = V(:,0:jb)^T w (no decision), result in w.cnew.

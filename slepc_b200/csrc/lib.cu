@@ -663,7 +663,6 @@ static void bv_free(b200_bv bv) {
   if (!bv) return;
   dev_free(bv->V);
   dev_free(bv->gs.st);
-  dev_free(bv->gs.coef);
   dev_free(bv->gs.cnew);
   dev_free(bv->gs.partials);
   dev_free(bv->coefbuf);
@@ -725,7 +724,7 @@ extern "C" b200_status b200_bv_create(int n, int m, void *stream, b200_bv *out) 
   bv->ldt = m + 1;
   const int sms = num_sms_host();
   bv->gs.num_sms = sms;
-  bv->gs.max_ctas = 2 * sms;  // the FP32-basis passes of the mixed solver run two CTAs per SM
+  bv->gs.max_ctas = sms;
   bv->red_len = sms * 8 > 4096 ? sms * 8 : 4096;
   bv->qbuf_len = (size_t)(m + 1) * (m + 1);
   bv->hpin_len = (size_t)(m + 1) * (m + 1) + 4 * (size_t)(m + 1) + 64;
@@ -734,7 +733,6 @@ extern "C" b200_status b200_bv_create(int n, int m, void *stream, b200_bv *out) 
   // final chunk round up to 16 bytes
   ok = ok && dev_malloc(&bv->V, sizeof(double) * ((size_t)bv->ld * (m + 1) + 32)) == cudaSuccess;
   ok = ok && dev_malloc(&bv->gs.st, sizeof(GsState)) == cudaSuccess;
-  ok = ok && dev_malloc(&bv->gs.coef, sizeof(double) * kMaxCols) == cudaSuccess;
   ok = ok && dev_malloc(&bv->gs.cnew, sizeof(double) * (kMaxCols + 1)) == cudaSuccess;
   ok = ok && dev_malloc(&bv->gs.partials, sizeof(double) * (size_t)(kMaxCols + 1) * 2 * sms) == cudaSuccess;
   ok = ok && dev_malloc(&bv->coefbuf, sizeof(double) * (size_t)bv->ldc * (m + 1)) == cudaSuccess;
@@ -751,7 +749,7 @@ extern "C" b200_status b200_bv_create(int n, int m, void *stream, b200_bv *out) 
   }
   cudaError_t e = cudaMemsetAsync(bv->V, 0, sizeof(double) * ((size_t)bv->ld * (m + 1) + 32), bv->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(bv->coefbuf, 0, sizeof(double) * (size_t)bv->ldc * (m + 1), bv->stream);
-  if (e == cudaSuccess) e = gs_state_reset(bv->gs, bv->eta, bv->stream);
+  if (e == cudaSuccess) e = gs_state_reset(bv->gs, bv->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(bv->stream);
   if (e != cudaSuccess) {
     bv_free(bv);
@@ -847,6 +845,7 @@ static b200_status bv_read_state(b200_bv bv, GsState *out) {
   B200_CUDA_CHECK(cudaMemcpyAsync(h, bv->gs.st, sizeof(GsState), cudaMemcpyDeviceToHost, bv->stream));
   B200_CUDA_CHECK(cudaStreamSynchronize(bv->stream));
   *out = *h;
+  if (out->err) B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->stream));
   if (out->err & kDevErrInnerProduct) {
     b200_set_last_error(__FILE__, __LINE__, "invalid inner product (negative self dot product)");
     return B200_ERR_INNER;
@@ -862,7 +861,6 @@ b200_status b200::bv_state(b200_bv bv, GsState *out) { return bv_read_state(bv, 
 
 // Orthogonalise column j against columns 0..j-1 (column variant).
 b200_status b200::bv_orth_column(b200_bv bv, int j, int normalize, double *H, double *norm, int *lindep) {
-  B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->eta, bv->stream));
   GsPassArgs a{};
   a.V = bv->V;
   a.ld = bv->ld;
@@ -876,7 +874,7 @@ b200_status b200::bv_orth_column(b200_bv bv, int j, int normalize, double *H, do
   a.step = -1;
   a.normalize = normalize;
   a.column = 1;
-  B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->stream));
+  B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->eta, true, bv->stream));
   if (H) {
     B200_CUDA_CHECK(cudaMemcpyAsync(bv->hpin + 64, a.hacc, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, bv->stream));
   }
@@ -903,7 +901,6 @@ extern "C" b200_status b200_bv_orthogonalize_vec(b200_bv bv, double *v, double *
   const int k = bv->k;
   // the vector is staged in the work column (column m) so every bulk copy stays inside the BV storage
   B200_CUDA_CHECK(copy_launch(col(bv, bv->m), v, bv->n, bv->stream));
-  B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->eta, bv->stream));
   GsPassArgs a{};
   a.V = bv->V;
   a.ld = bv->ld;
@@ -915,7 +912,7 @@ extern "C" b200_status b200_bv_orthogonalize_vec(b200_bv bv, double *v, double *
   a.step = -1;
   a.normalize = 0;
   a.column = 0;
-  B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->stream));
+  B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->eta, true, bv->stream));
   B200_CUDA_CHECK(copy_launch(v, col(bv, bv->m), bv->n, bv->stream));
   if (H && k > 0)
     B200_CUDA_CHECK(cudaMemcpyAsync(bv->hpin + 64, bv->hvec, sizeof(double) * k, cudaMemcpyDeviceToHost, bv->stream));
@@ -1068,7 +1065,6 @@ b200_status b200::bv_orthogonalize_block(b200_bv bv) {
   if (nc <= 0) return B200_OK;
   B200_CHECK(bv_reserve(bv, (size_t)3 * nc, 0));
   for (int j = bv->l; j < bv->k; ++j) {
-    B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->eta, bv->stream));
     GsPassArgs a{};
     a.V = bv->V;
     a.ld = bv->ld;
@@ -1080,7 +1076,7 @@ b200_status b200::bv_orthogonalize_block(b200_bv bv) {
     a.step = -1;
     a.normalize = 1;
     a.column = 1;
-    B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->stream));
+    B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->eta, true, bv->stream));
     B200_CUDA_CHECK(gs_record_launch(bv->gs, bv->qbuf + 3 * (size_t)(j - bv->l), bv->stream));
   }
   B200_CUDA_CHECK(
@@ -1088,6 +1084,7 @@ b200_status b200::bv_orthogonalize_block(b200_bv bv) {
   B200_CUDA_CHECK(cudaStreamSynchronize(bv->stream));
   for (int c = 0; c < nc; ++c) {
     const int err = (int)bv->hpin[3 * c + 2];
+    if (err) B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->stream));
     if (err & kDevErrInnerProduct) {
       b200_set_last_error(__FILE__, __LINE__, "invalid inner product (negative self dot product)");
       return B200_ERR_INNER;
@@ -1110,7 +1107,6 @@ b200_status b200::bv_orthonormalize_vecs(b200_bv bv, double *const *vecs, int co
   B200_CHECK(bv_reserve(bv, (size_t)3 * count, 0));
   for (int i = 0; i < count; ++i) {
     B200_CUDA_CHECK(copy_launch(col(bv, bv->m), vecs[i], bv->n, bv->stream));
-    B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->eta, bv->stream));
     GsPassArgs a{};
     a.V = bv->V;
     a.ld = bv->ld;
@@ -1122,7 +1118,7 @@ b200_status b200::bv_orthonormalize_vecs(b200_bv bv, double *const *vecs, int co
     a.step = -1;
     a.normalize = 1;
     a.column = 0;
-    B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->stream));
+    B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->eta, true, bv->stream));
     B200_CUDA_CHECK(copy_launch(vecs[i], col(bv, bv->m), bv->n, bv->stream));
     B200_CUDA_CHECK(gs_record_launch(bv->gs, bv->qbuf + 3 * (size_t)i, bv->stream));
   }
@@ -1131,6 +1127,7 @@ b200_status b200::bv_orthonormalize_vecs(b200_bv bv, double *const *vecs, int co
   B200_CUDA_CHECK(cudaStreamSynchronize(bv->stream));
   for (int i = 0; i < count; ++i) {
     const int err = (int)bv->hpin[3 * i + 2];
+    if (err) B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->stream));
     if (err) B200_DEV_ERR("a Gram-Schmidt kernel reported a device-side error");
     if (!(bv->hpin[3 * i] > 0.0) || bv->hpin[3 * i + 1] != 0.0) *breakdown = 1;
   }
@@ -1589,7 +1586,6 @@ struct RunTimer {
 static b200_status bv_lanczos(b200_bv bv, b200_mat A, int k, int *m, double *alpha, double *beta_h, double *beta,
                               int *breakdown, RunTimer *timer, GsState *st_out) {
   const int m0 = *m;
-  B200_CUDA_CHECK(gs_state_reset(bv->gs, bv->eta, bv->stream));
   const bool timing = timer && timer->on;
   if (timing) {
     timer->reserve((size_t)4 * (m0 - k) + 4);
@@ -1599,7 +1595,8 @@ static b200_status bv_lanczos(b200_bv bv, b200_mat A, int k, int *m, double *alp
     cudaEvent_t e0 = timing ? timer->next() : nullptr, e1 = timing ? timer->next() : nullptr;
     cudaEvent_t e2 = timing ? timer->next() : nullptr, e3 = timing ? timer->next() : nullptr;
     if (e0) cudaEventRecord(e0, bv->stream);
-    B200_CUDA_CHECK(mat_spmv(A, col(bv, j), col(bv, j + 1), bv->stream, bv->gs.st, j));
+    // the first step of a run is not gated on the control block (it still holds the previous run)
+    B200_CUDA_CHECK(mat_spmv(A, col(bv, j), col(bv, j + 1), bv->stream, j == k ? nullptr : bv->gs.st, j));
     if (e1) cudaEventRecord(e1, bv->stream);
     GsPassArgs a{};
     a.V = bv->V;
@@ -1615,7 +1612,7 @@ static b200_status bv_lanczos(b200_bv bv, b200_mat A, int k, int *m, double *alp
     a.normalize = 1;
     a.column = 1;
     if (e2) cudaEventRecord(e2, bv->stream);
-    B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->stream));
+    B200_CUDA_CHECK(gs_orthogonalize_launch(a, bv->gs, bv->eta, j == k, bv->stream));
     if (e3) cudaEventRecord(e3, bv->stream);
   }
   // one device-to-host copy of T and of the control block

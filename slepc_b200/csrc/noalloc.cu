@@ -31,11 +31,11 @@
 namespace b200 {
 namespace {
 
-// Capacity of the scratch: the control block, the coefficient vectors and the
-// per-CTA partial dot products of up to kNoAllocMaxCtas CTAs.
+// Capacity of the scratch: the control block, the reduced dot and the per-CTA
+// partial dot products of up to kNoAllocMaxCtas CTAs, for two passes.
 constexpr int kNoAllocMaxCtas = 160;
 constexpr size_t kScratchDoubles =
-    (sizeof(GsState) + 7) / 8 + 32 + kMaxCols + (kMaxCols + 1) + (size_t)(kMaxCols + 1) * kNoAllocMaxCtas;
+    (sizeof(GsState) + 7) / 8 + 32 + (kMaxCols + 1) + 2 * (size_t)(kMaxCols + 1) * kNoAllocMaxCtas;
 
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
@@ -107,13 +107,11 @@ extern "C" b200_status b200_orthogonalize_column_noalloc(int n, int ld, int ncol
   double *base = nullptr;
   B200_CUDA_CHECK(scratch_address(&base));
 
-  // carve the scratch: control block, coefficients, reduced dot, per-CTA partials
+  // carve the scratch: control block, reduced dot, per-CTA partials
   GsWork w{};
   double *q = base;
   w.st = reinterpret_cast<GsState *>(q);
   q += (sizeof(GsState) + 7) / 8 + 32;
-  w.coef = q;
-  q += kMaxCols;
   w.cnew = q;
   q += kMaxCols + 1;
   w.partials = q;
@@ -124,7 +122,7 @@ extern "C" b200_status b200_orthogonalize_column_noalloc(int n, int ld, int ncol
   w.max_ctas = sms < kNoAllocMaxCtas ? sms : kNoAllocMaxCtas;
 
   // the control block carries over from the last call: start it from zero
-  B200_CUDA_CHECK(gs_state_reset(w, 0.7071, s));
+  B200_CUDA_CHECK(gs_state_reset(w, s));
   GsPassArgs a{};
   a.V = V;
   a.ld = ld;
@@ -138,7 +136,7 @@ extern "C" b200_status b200_orthogonalize_column_noalloc(int n, int ld, int ncol
   a.step = -1;
   a.normalize = 0;
   a.column = 1;
-  B200_CUDA_CHECK(gs_orthogonalize_launch(a, w, s));
+  B200_CUDA_CHECK(gs_orthogonalize_launch(a, w, 0.7071, true, s));
   GsState st;
   B200_CUDA_CHECK(cudaMemcpyAsync(&st, w.st, sizeof(GsState), cudaMemcpyDeviceToHost, s));
   B200_CUDA_CHECK(cudaStreamSynchronize(s));

@@ -64,7 +64,7 @@ def gs(args, torch):
     ms /= args.reps
     # three streamed passes (dot; update+dot; update+scale) of j basis columns plus w, and two writes of w
     algo = 8 * n * (3 * (j + 1) + 2)
-    return {"kernel": "gs_pass_kernel x3 (one column, DGKS refined)", "n": n, "j": j, "ms": ms,
+    return {"kernel": "gs_column_kernel (one column, DGKS refined)", "n": n, "j": j, "ms": ms,
             "algorithmic_bytes": algo, "GBps": algo / (ms * 1e-3) / 1e9, "norm": nrm, "ld": ld}
 
 
