@@ -49,6 +49,7 @@ struct GsState {
   int halt;             // set when a Lanczos run broke down: later steps are skipped
   int halt_step;        // Lanczos step index at which the breakdown happened
   int err;              // DeviceError bits
+  unsigned int run_ticket, run_exit;  // barrier and exit counters of a whole-run launch (zero between launches)
   int passes;           // passes done since the start of the run
   double beta_out;      // norm returned to the caller (BVOrthonormalizeColumn's norm)
   unsigned long long bytes;  // algorithmic bytes moved by those passes

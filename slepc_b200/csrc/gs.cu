@@ -21,6 +21,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <atomic>
+
 #include "common.h"
 #include "kernels.h"
 
@@ -32,6 +34,7 @@ constexpr int kConsumers = kConsumerWarps * 32;  // 256 consumer threads
 constexpr int kThreads = kConsumers + 32;        // + one producer warp issuing the tile loads
 constexpr int kPartCols = 32;                    // most basis columns a consumer lane holds in registers
 constexpr int kMaxStages = 8;
+constexpr double kDefTol = 10.0 * 2.220446049250313e-16;  // BV deftol = 10*PETSC_MACHINE_EPSILON (bvfunc.c:184)
 constexpr size_t kStageBudget = 192 * 1024;      // bytes of all stages together
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -106,13 +109,25 @@ __device__ __forceinline__ double lane_column_sums(const double (&acc)[CPW], int
   return v[0];
 }
 
+// Lane l returns the sum over the lanes of d[l / 8]: two halving exchanges and a tree, 6 shuffles for four
+// columns (the shuffles, not the additions, bound a short dot: 20 a tree each).
+__device__ __forceinline__ double quad_sum(const double (&d)[4], int lane) {
+  const bool up = (lane & 16) != 0, odd = (lane & 8) != 0;
+  const double a0 = up ? d[2] : d[0], a1 = up ? d[3] : d[1], b0 = up ? d[0] : d[2], b1 = up ? d[1] : d[3];
+  const double e0 = a0 + __shfl_xor_sync(0xffffffffu, b0, 16), e1 = a1 + __shfl_xor_sync(0xffffffffu, b1, 16);
+  double v = (odd ? e1 : e0) + __shfl_xor_sync(0xffffffffu, odd ? e0 : e1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 struct ColumnParams {
   GsPassArgs a;
   GsState *st;
   double *cnew;
   double *partials;  // two buffers of G x (jb + 1) per-CTA dots, by parity of the pass
   double eta;
-  double deftol;     // BV deftol = 10*PETSC_MACHINE_EPSILON (bvfunc.c:184)
+  double deftol;
   int fresh;         // start of a run: the control block's counters and halt flag are replaced (not its error bits)
   int plain_dot;     // plain BVDotVec: one DOT, no decision
   int parts;         // warps that share a group of 32 rows (1, 2, 4, 8): each owns 1/parts of the columns
@@ -453,6 +468,529 @@ __global__ void __launch_bounds__(kThreads, 1) gs_column_kernel(ColumnParams p, 
   }
 }
 
+// ---------------------------------------------------------------- a whole Lanczos run in one launch
+//
+// BVMatLanczos for a basis that fits the chip's shared memory: every CTA owns a contiguous range of
+// 32-row slices of the sliced-ELL operator and keeps its rows of all the run's basis columns in shared
+// memory, so a column costs no launch and no basis traffic: SpMV of its rows, then the passes of
+// gs_column_kernel with the same DGKS decisions, an exchange of the CTAs' dots after each DOT and a
+// barrier when the new column is complete.  Two forms:
+//   * gs_cluster_run_kernel, the smallest: one 16-CTA cluster, the exchanges and the gathered x through
+//     distributed shared memory;
+//   * gs_run_kernel: up to one CTA per SM, the exchanges and x through L2.
+// What bounds both is a chain of latencies (exchange, decision, SpMV gathers), and beside it the issue
+// slots: a phase is a few hundred instructions per warp, so the loops keep their indices in 32 bits, take
+// no divisions and give every warp one share.
+// Measured (BVMatLanczos on 2-D Laplacians, whole calls; column by column / one CTA per SM / one cluster):
+// n = 3,660 columns 0..30 583 / 356 / 232 us; n = 10,000 columns 16..32 373 / 221 / 195; n = 14,400 columns
+// 0..20 428 / 254 / 192; n = 40,000 columns 0..40 1,031 / 592 / -; n = 65,000 columns 0..20 508 / 320 / -.
+// So the cluster runs wherever its shared memory holds the basis, then one CTA per SM wherever that does.
+constexpr int kRunWarps = 16;
+constexpr int kRunThreads = kRunWarps * 32;
+constexpr int kRunCached = 8;                   // entries per row of the operator held in registers
+constexpr size_t kRunSmem = 184 * 1024;         // shared memory for the basis rows, w and its partial updates
+
+struct RunParams {
+  double *V;
+  int ld, n, k, m;
+  double *coefbuf;  // column j + 1 of the coefficient buffer gets the coefficients of column j + 1
+  int ldc;
+  double *T;
+  int ldt;
+  GsState *st;
+  ulonglong2 *slots;         // two buffers of G x (jb + 1) {partial dot, epoch}
+  unsigned long long epoch;  // epochs of this run start above it (no earlier run on these slots used them)
+  double eta, deftol;
+  int nslices, spc;          // slices of the operator, slices per CTA
+  const long long *off;
+  const int *width;
+  const int *cols;
+};
+
+// What the passes of a run share with the CTA's threads.
+struct RunPass {
+  int action, lindep;
+  double scale, nrm;
+};
+
+// sum over c < nc of v[c R] coef[c]; coef 16-byte aligned
+__device__ __forceinline__ double run_row_sum(const double *v, int R, const double *coef, int nc) {
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+  int c = 0;
+#pragma unroll 2
+  for (; c + 4 <= nc; c += 4, v += 4 * R) {
+    const double2 ca = *reinterpret_cast<const double2 *>(coef + c), cb = *reinterpret_cast<const double2 *>(coef + c + 2);
+    s0 = fma(v[0], ca.x, s0);
+    s1 = fma(v[R], ca.y, s1);
+    s2 = fma(v[2 * R], cb.x, s2);
+    s3 = fma(v[3 * R], cb.y, s3);
+  }
+  for (; c < nc; ++c, v += R) s0 = fma(v[0], coef[c], s0);
+  return (s0 + s1) + (s2 + s3);
+}
+
+// UPDATE and SCALE of the CTA's rows.  With parts = 1 << lp warps to a slice (lp > 0: at most 16 slices a
+// CTA, one share per warp) the parts of the columns meet in ups; with one warp to a slice a lane finishes
+// its row by itself.
+__device__ __forceinline__ void run_update(const double *Vs, double *ws, double *ups, const double *coef, int jb, int R,
+                                           int spc, int lp, int slice, int part, bool update, double scale) {
+  const int lane = threadIdx.x & 31;
+  if (lp > 0) {
+    if (update) {
+      if (part < (1 << lp)) {
+        const int q = (((jb + (1 << lp) - 1) >> lp) + 1) & ~1, c0 = part * q;  // even: aligned coefficient pairs
+        ups[part * R + 32 * slice + lane] =
+            run_row_sum(Vs + c0 * R + 32 * slice + lane, R, coef + c0, min(q, jb - c0));
+      }
+      __syncthreads();
+    }
+    for (int r = threadIdx.x; r < R; r += kRunThreads) {
+      double tot = 0.0;
+      if (update)
+        for (int q = 0; q < (1 << lp); ++q) tot += ups[q * R + r];
+      ws[r] = (ws[r] - tot) * scale;
+    }
+  } else {
+    for (int s = slice; s < spc; s += kRunWarps) {
+      const int r = 32 * s + lane;
+      const double tot = update ? run_row_sum(Vs + r, R, coef, jb) : 0.0;
+      ws[r] = (ws[r] - tot) * scale;
+    }
+  }
+  __syncthreads();
+}
+
+// Lane l returns column 4 cg + l / 8 of the dots of w with the basis columns (column jb is w itself) over
+// the rows [ra, rb) of the CTA.
+__device__ __forceinline__ double run_dot4(const double *Vs, const double *ws, int jb, int R, int cg, int ra, int rb) {
+  const int lane = threadIdx.x & 31;
+  const double *v[4];
+  double d[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = 4 * cg + q < jb ? Vs + (4 * cg + q) * R : ws;
+#pragma unroll 2
+  for (int r = ra + lane; r < rb; r += 32) {
+    const double wv = ws[r];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) d[q] = fma(v[q][r], wv, d[q]);
+  }
+  return quad_sum(d, lane);
+}
+
+// The decision after an exchange, by warp 0 (d stays in its registers), published for the CTA.
+__device__ __forceinline__ void run_decide(Decision &d, const ColumnParams &cp, const double *cnew_s, double *coef_s,
+                                           double *hsum, RunPass *pass) {
+  const int lane = threadIdx.x & 31;
+  decide(d, cp, cnew_s, coef_s, hsum, lane);
+  if (lane == 0) {
+    pass->action = d.action;
+    pass->scale = d.scale;
+    if (d.stage == kStageDone) {
+      pass->lindep = d.lindep;
+      pass->nrm = d.nrm;
+    }
+  }
+}
+
+// The outputs of a finished column: coefficients, alpha and beta, error bits.
+__device__ __forceinline__ void run_column_out(const RunParams &p, int j, const double *hsum, const RunPass &pass) {
+  const int jb = j + 1;
+  double *h = p.coefbuf + (size_t)jb * p.ldc;
+  for (int c = threadIdx.x; c < jb; c += kRunThreads) h[c] = hsum[c];
+  if (threadIdx.x == 0) {
+    const double beta = pass.lindep ? 0.0 : pass.nrm;
+    h[jb] = beta;
+    p.T[j] = hsum[jb - 1];
+    p.T[p.ldt + j] = beta;
+  }
+}
+
+// {value, epoch} of one CTA's partial dot.  The pair is stored and loaded as one 16-byte access (single-copy
+// atomic for .b128), so a reader that finds the epoch it waits for has the value too: the exchange after a
+// DOT needs neither a fence nor an arrival counter.
+__device__ __forceinline__ void slot_store(ulonglong2 *slot, double v, unsigned long long epoch) {
+  asm volatile("{\n .reg .b128 q;\n mov.b128 q, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], q;\n}\n" ::"l"(slot),
+               "l"(__double_as_longlong(v)), "l"(epoch)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 slot_load(const ulonglong2 *slot) {
+  ulonglong2 r;
+  asm volatile("{\n .reg .b128 q;\n ld.relaxed.gpu.global.b128 q, [%2];\n mov.b128 {%0, %1}, q;\n}\n"
+               : "=l"(r.x), "=l"(r.y)
+               : "l"(slot)
+               : "memory");
+  return r;
+}
+
+template <typename VT>
+__global__ void __launch_bounds__(kRunThreads, 1) gs_run_kernel(RunParams p, const VT *__restrict__ sval) {
+  extern __shared__ __align__(16) double run_smem[];
+  __shared__ __align__(16) double coef_s[kMaxCols + 1];
+  __shared__ double cnew_s[kMaxCols + 1], hsum[kMaxCols + 1];
+  __shared__ double red[kRunWarps][kMaxCols + 1];
+  __shared__ RunPass ps;
+  __shared__ int grid_ok;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" :::);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = gridDim.x, n = p.n, spc = p.spc, R = 32 * spc;
+  const int r0 = blockIdx.x * R, rows = min(R, n - r0);
+  const int lp = 31 - __clz(kRunWarps / spc);  // parts of the columns in an update: 1 << lp warps to a slice
+  const int slice = warp % spc, part = warp / spc;
+  double *ws = run_smem;       // w of the CTA's rows
+  double *ups = ws + R;        // partial updates [part][row]
+  double *Vs = ups + (R << lp);  // basis columns [column][row]
+  for (int c = 0; c <= p.k; ++c)
+    for (int r = tid; r < R; r += kRunThreads) Vs[c * R + r] = r < rows ? p.V[(size_t)c * p.ld + r0 + r] : 0.0;
+  // the operator's entries of this lane's row: the first kRunCached stay in registers for the run
+  const int sl = blockIdx.x * spc + warp;
+  const bool has_slice = warp < spc && sl < p.nslices;
+  const int wid = has_slice ? p.width[sl] : 0;
+  const long long base = has_slice ? p.off[sl] + lane : 0;
+  int cc[kRunCached];
+  VT aa[kRunCached];
+#pragma unroll
+  for (int u = 0; u < kRunCached; ++u) {
+    cc[u] = u < wid ? p.cols[base + 32ll * u] : -1;
+    aa[u] = u < wid ? sval[base + 32ll * u] : VT(0);
+  }
+  if (tid == 0) grid_ok = 1;
+  unsigned target = 0;
+  // Grid barrier: the arrivals of all CTAs bring the word to the next multiple of G.  False (for the whole
+  // CTA) after kSpinLimit polls.
+  auto grid_sync = [&]() -> bool {
+    target += (unsigned)G;
+    __syncthreads();
+    if (tid == 0) {
+      asm volatile("fence.acq_rel.gpu;\n red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(&p.st->run_ticket) : "memory");
+      int ok = 0;
+      for (long long it = 0; it < kSpinLimit && !ok; ++it) {
+        unsigned now;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&p.st->run_ticket) : "memory");
+        ok = (int)(now - target) >= 0;
+      }
+      grid_ok = ok;
+    }
+    __syncthreads();
+    return grid_ok != 0;
+  };
+
+  ColumnParams cp;  // what the decision reads
+  cp.eta = p.eta;
+  cp.deftol = p.deftol;
+  cp.a.normalize = 1;
+  cp.a.column = 1;
+  Decision d;
+  unsigned npass = 0;
+  unsigned long long epoch = p.epoch, bytes = 0;
+  bool ok = true;
+  int halt = 0, halt_step = -1, errs = 0;
+  double beta = 0.0;
+  for (int j = p.k; j < p.m && ok && !halt; ++j) {
+    const int jb = j + 1, ldp = jb + 1;
+    const double *x = p.V + (size_t)j * p.ld;  // written by every CTA: read through L2
+    if (warp < spc) {
+      double sacc = 0.0;
+      double xv[kRunCached];
+#pragma unroll
+      for (int u = 0; u < kRunCached; ++u) xv[u] = cc[u] >= 0 ? __ldcg(x + cc[u]) : 0.0;
+#pragma unroll
+      for (int u = 0; u < kRunCached; ++u)
+        if (cc[u] >= 0) sacc = __dadd_rn(sacc, __dmul_rn((double)aa[u], xv[u]));
+      for (int u = kRunCached; u < wid; ++u) {
+        const int c = p.cols[base + 32ll * u];
+        if (c >= 0) sacc = __dadd_rn(sacc, __dmul_rn((double)sval[base + 32ll * u], __ldcg(x + c)));
+      }
+      ws[32 * warp + lane] = sacc;  // rows past n have no entries
+    }
+    d = Decision{kStageDotOfPass, 0, kActDot, 0, 0, 0.0, 0.0, 1.0};
+    cp.a.jb = jb;
+    int action = kActDot;
+    double scale = 1.0;
+    __syncthreads();
+    for (;;) {
+      const bool update = (action & kActUpdate) != 0, rewrite = (action & (kActUpdate | kActScale)) != 0;
+      const bool dot = (action & kActDot) != 0;
+      ++npass;
+      bytes += (unsigned long long)n * 8ull * ((update || dot ? jb : 0) + 1 + (rewrite ? 1 : 0));
+      if (rewrite) run_update(Vs, ws, ups, coef_s, jb, R, spc, lp, slice, part, update, scale);
+      if (!dot) break;
+      ulonglong2 *pb = p.slots + (size_t)(epoch & 1) * G * ldp;
+      ++epoch;
+      for (int cg = warp; 4 * cg <= jb; cg += kRunWarps) {
+        const double mine = run_dot4(Vs, ws, jb, R, cg, 0, R);
+        const int c = 4 * cg + (lane >> 3);
+        if ((lane & 7) == 0 && c <= jb) slot_store(pb + blockIdx.x * ldp + c, mine, epoch);
+      }
+      // Fixed-order sum over the CTAs: warp w adds CTAs w, w + 16, ... with one column per lane, up to eight
+      // loads in flight, each repeated until it brings this exchange's epoch.
+      bool arrived = true;
+      for (int c = lane; c <= jb; c += 32) {
+        double sacc = 0.0;
+        for (int b0 = warp; b0 < G; b0 += 8 * kRunWarps) {
+          ulonglong2 r[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (b0 + u * kRunWarps < G) r[u] = slot_load(pb + (b0 + u * kRunWarps) * ldp + c);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (b0 + u * kRunWarps < G) {
+              for (long long it = 0; r[u].y != epoch && arrived; ++it) {
+                r[u] = slot_load(pb + (b0 + u * kRunWarps) * ldp + c);
+                if (it >= kSpinLimit) arrived = false;
+              }
+              sacc += __longlong_as_double(r[u].x);
+            }
+        }
+        red[warp][c] = sacc;
+      }
+      if (!arrived) grid_ok = 0;
+      __syncthreads();
+      ok = grid_ok != 0;
+      if (!ok) break;
+      if (warp == 0) {
+        for (int c = lane; c <= jb; c += 32) {
+          double t[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) t[q] = (red[q][c] + red[q + 4][c]) + (red[q + 8][c] + red[q + 12][c]);
+          cnew_s[c] = (t[0] + t[1]) + (t[2] + t[3]);
+        }
+        __syncwarp();
+        run_decide(d, cp, cnew_s, coef_s, hsum, &ps);
+        errs |= d.err;
+      }
+      __syncthreads();
+      action = ps.action;
+      scale = ps.scale;
+      if (action == kActNone) break;
+    }
+    if (!ok) break;
+    // the new column: into the basis rows of this CTA and into V, where every CTA gathers it
+    double *vn = p.V + (size_t)jb * p.ld + r0;
+    for (int r = tid; r < R; r += kRunThreads) {
+      Vs[jb * R + r] = ws[r];
+      if (r < rows) __stcg(vn + r, ws[r]);
+    }
+    beta = ps.nrm;
+    if (blockIdx.x == 0) run_column_out(p, j, hsum, ps);
+    if (ps.lindep) {
+      halt = 1;
+      halt_step = j;
+    } else if (j + 1 < p.m) {
+      ok = grid_sync();
+    }
+  }
+  if (tid == 0) {
+    if (!ok) atomicOr(&p.st->err, (int)kDevErrTimeout);
+    if (blockIdx.x == 0 && ok) {
+      if (errs) atomicOr(&p.st->err, errs);
+      p.st->beta_out = beta;
+      p.st->lindep = halt;
+      p.st->halt = halt;
+      p.st->halt_step = halt_step;
+      p.st->passes = (int)npass;
+      p.st->bytes = bytes;
+    }
+    // the last CTA to leave clears the barrier word for the next run
+    __threadfence();
+    if (atomicAdd(&p.st->run_exit, 1u) == (unsigned)(G - 1)) {
+      p.st->run_ticket = 0;
+      p.st->run_exit = 0;
+    }
+  }
+}
+
+// ---- the cluster form
+constexpr int kClusterCtas = 16;
+constexpr int kRowParts = 2;       // the rows of a dot are split in two, so that a short basis feeds all warps
+constexpr int kClusterSlices = 2;  // slices of the operator a warp applies
+
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t cta) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ double cluster_load(uint32_t addr) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+  return v;
+}
+// Store to another CTA's shared memory that counts its bytes on that CTA's mbarrier: the receiver's wait
+// for the bytes is the whole exchange (a store followed by the cluster barrier takes twice as long).
+__device__ __forceinline__ void cluster_store_tx(uint32_t addr, double v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Shared doubles of a CTA: basis rows, w, partial updates, dot exchange.
+__host__ __device__ inline size_t cluster_run_doubles(int spc, int m) {
+  const int parts = spc <= kRunWarps / 2 ? kRunWarps / spc : 1;
+  return (size_t)32 * spc * (m + 1 + 1 + parts) + (size_t)2 * kClusterCtas * kRowParts * (m + 1);
+}
+
+template <typename VT>
+__global__ void __launch_bounds__(kRunThreads, 1) gs_cluster_run_kernel(RunParams p, const VT *__restrict__ sval) {
+  extern __shared__ __align__(16) double run_smem[];
+  __shared__ __align__(16) double coef_s[kMaxCols + 1];
+  __shared__ double cnew_s[kMaxCols + 1], hsum[kMaxCols + 1];
+  __shared__ __align__(8) uint64_t bars[2];  // bytes of an exchange, by its parity
+  __shared__ RunPass ps;
+  __shared__ volatile int gave_up, stop;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" :::);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = p.n, spc = p.spc, R = 32 * spc, rank = blockIdx.x;
+  const int r0 = rank * R, rows = min(R, n - r0);  // negative for a CTA past the last row
+  const int lp = spc <= kRunWarps / 2 ? 31 - __clz(kRunWarps / spc) : 0;
+  const int slice = lp ? warp % spc : warp, part = lp ? warp / spc : 0;
+  double *Vs = run_smem;                  // basis rows [column][row]
+  double *ws = Vs + (p.m + 1) * R;        // w of the CTA's rows
+  double *xch = ws + R;                   // two buffers of [CTA and row part][column] dots
+  double *ups = xch + 2 * kClusterCtas * kRowParts * (p.m + 1);  // partial updates [part][row]
+  if (tid == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    fence_mbar_init();
+    gave_up = 0;
+    stop = 0;
+  }
+  for (int c = 0; c <= p.k; ++c)
+    for (int r = tid; r < R; r += kRunThreads) Vs[c * R + r] = r < rows ? p.V[(size_t)c * p.ld + r0 + r] : 0.0;
+  // the operator's entries of this lane's rows (slices warp and warp + 16 of the CTA): the first kRunCached
+  // of a row stay in registers for the run, a column as the cluster address of its basis row
+  const uint32_t vs0 = smem_u32(Vs);
+  uint32_t ca[kClusterSlices][kRunCached];
+  VT aa[kClusterSlices][kRunCached];
+  int wid[kClusterSlices];
+  long long base[kClusterSlices];
+  auto address = [&](int c) { return c >= 0 ? cluster_map(vs0 + 8u * (uint32_t)(c % R), (uint32_t)(c / R)) : 0u; };
+#pragma unroll
+  for (int h = 0; h < kClusterSlices; ++h) {
+    const int ls = warp + h * kRunWarps, sl = rank * spc + ls;
+    const bool has = ls < spc && sl < p.nslices;
+    wid[h] = has ? p.width[sl] : 0;
+    base[h] = has ? p.off[sl] + lane : 0;
+#pragma unroll
+    for (int u = 0; u < kRunCached; ++u) {
+      ca[h][u] = u < wid[h] ? address(p.cols[base[h] + 32ll * u]) : 0u;
+      aa[h][u] = u < wid[h] ? sval[base[h] + 32ll * u] : VT(0);
+    }
+  }
+  ColumnParams cp;  // what the decision reads
+  cp.eta = p.eta;
+  cp.deftol = p.deftol;
+  cp.a.normalize = 1;
+  cp.a.column = 1;
+  Decision d;
+  unsigned npass = 0, exchange = 0;
+  unsigned long long bytes = 0;
+  int halt = 0, halt_step = -1, errs = 0;
+  double beta = 0.0;
+  cluster_sync();  // every CTA's basis rows are loaded and its mbarriers live
+  for (int j = p.k; j < p.m && !halt; ++j) {
+    const int jb = j + 1, ldp = jb + 1;
+    const uint32_t xoff = 8u * (uint32_t)j * (uint32_t)R;  // column j of any CTA's basis rows
+#pragma unroll
+    for (int h = 0; h < kClusterSlices; ++h) {
+      const int ls = warp + h * kRunWarps;
+      if (ls < spc) {
+        double xv[kRunCached], sacc = 0.0;
+#pragma unroll
+        for (int u = 0; u < kRunCached; ++u) xv[u] = ca[h][u] ? cluster_load(ca[h][u] + xoff) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kRunCached; ++u)
+          if (ca[h][u]) sacc = __dadd_rn(sacc, __dmul_rn((double)aa[h][u], xv[u]));
+        for (int u = kRunCached; u < wid[h]; ++u) {
+          const uint32_t a = address(p.cols[base[h] + 32ll * u]);
+          if (a) sacc = __dadd_rn(sacc, __dmul_rn((double)sval[base[h] + 32ll * u], cluster_load(a + xoff)));
+        }
+        ws[32 * ls + lane] = sacc;  // rows past n have no entries
+      }
+    }
+    d = Decision{kStageDotOfPass, 0, kActDot, 0, 0, 0.0, 0.0, 1.0};
+    cp.a.jb = jb;
+    int action = kActDot;
+    double scale = 1.0;
+    __syncthreads();
+    for (;;) {
+      const bool update = (action & kActUpdate) != 0, rewrite = (action & (kActUpdate | kActScale)) != 0;
+      const bool dot = (action & kActDot) != 0;
+      ++npass;
+      bytes += (unsigned long long)n * 8ull * ((update || dot ? jb : 0) + 1 + (rewrite ? 1 : 0));
+      if (rewrite) run_update(Vs, ws, ups, coef_s, jb, R, spc, lp, slice, part, update, scale);
+      if (!dot) break;
+      // (four columns, half of the rows) shares over the warps; each sum goes to every CTA of the cluster
+      const int buf = exchange & 1;
+      double *xb = xch + buf * kClusterCtas * kRowParts * (p.m + 1);
+      if (tid == 0) mbar_arrive_expect_tx(&bars[buf], (uint32_t)(kClusterCtas * kRowParts * ldp * 8));
+      const uint32_t bar = smem_u32(&bars[buf]);
+      for (int it = warp; 4 * (it / kRowParts) <= jb; it += kRunWarps) {
+        const int cg = it / kRowParts, rp = it % kRowParts;
+        const double mine = run_dot4(Vs, ws, jb, R, cg, rp ? 32 * (spc / 2) : 0, rp ? R : 32 * (spc / 2));
+        const int c = 4 * cg + (lane >> 3);
+        if (c <= jb) {
+          const uint32_t slot = smem_u32(xb + (rank * kRowParts + rp) * (p.m + 1) + c);
+#pragma unroll
+          for (int t = 0; t < kClusterCtas / 8; ++t) {
+            const uint32_t to = (lane & 7) + 8 * t;
+            cluster_store_tx(cluster_map(slot, to), mine, cluster_map(bar, to));
+          }
+        }
+      }
+      if (warp == 0) {
+        mbar_wait_bounded(&bars[buf], (exchange >> 1) & 1, &gave_up);
+        for (int c = lane; c <= jb; c += 32) {
+          const double *x = xb + c;
+          double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+          for (int b = 0; b < kClusterCtas * kRowParts; ++b) t[b & 3] += x[b * (p.m + 1)];
+          cnew_s[c] = (t[0] + t[1]) + (t[2] + t[3]);
+        }
+        __syncwarp();
+        run_decide(d, cp, cnew_s, coef_s, hsum, &ps);
+        errs |= d.err;
+      }
+      ++exchange;
+      __syncthreads();
+      action = ps.action;
+      scale = ps.scale;
+      if (action == kActNone || gave_up) break;
+    }
+    // the new column: into the basis rows, where the cluster gathers it, and into V
+    double *vn = p.V + (size_t)jb * p.ld + r0;
+    for (int r = tid; r < R; r += kRunThreads) {
+      Vs[jb * R + r] = ws[r];
+      if (r < rows) vn[r] = ws[r];
+    }
+    beta = ps.nrm;
+    if (rank == 0) run_column_out(p, j, hsum, ps);
+    if (ps.lindep) {
+      halt = 1;
+      halt_step = j;
+    }
+    // a CTA that gave up a wait stops the whole cluster here, so that none sends to a CTA that has left
+    if (gave_up && tid < kClusterCtas)
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_map(smem_u32((const void *)&stop), tid)), "r"(1) : "memory");
+    cluster_sync();  // column j + 1 is complete; after the last column, no CTA leaves while another reads it
+    if (stop) break;
+  }
+  if (tid == 0 && gave_up) atomicOr(&p.st->err, (int)kDevErrTimeout);
+  if (rank == 0 && tid == 0) {
+    if (errs) atomicOr(&p.st->err, errs);
+    p.st->beta_out = beta;
+    p.st->lindep = halt;
+    p.st->halt = halt;
+    p.st->halt_step = halt_step;
+    p.st->passes = (int)npass;
+    p.st->bytes = bytes;
+  }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     void *ptr = nullptr;
@@ -527,7 +1065,7 @@ cudaError_t launch_column(const GsPassArgs &a, const GsWork &w, double eta, int 
   p.cnew = w.cnew;
   p.partials = w.partials;
   p.eta = eta;
-  p.deftol = 10.0 * 2.220446049250313e-16;
+  p.deftol = kDefTol;
   p.fresh = fresh;
   p.plain_dot = plain_dot;
   p.parts = column_parts(a.jb);
@@ -544,6 +1082,75 @@ cudaError_t launch_column(const GsPassArgs &a, const GsWork &w, double eta, int 
   if (q <= 24) return launch_column_t<24>(p, G, stream);
   if (q <= 28) return launch_column_t<28>(p, G, stream);
   return launch_column_t<32>(p, G, stream);
+}
+
+template <typename VT>
+cudaError_t launch_run(RunParams &p, const void *vals, int G, size_t smem, cudaStream_t stream) {
+  cudaError_t e = allow_max_dynamic_smem(gs_run_kernel<VT>);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)G);
+  cfg.blockDim = dim3(kRunThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  e = cudaLaunchKernelEx(&cfg, gs_run_kernel<VT>, p, static_cast<const VT *>(vals));
+  count_launch();
+  return e;
+}
+
+// The cluster form where one fits; cudaErrorNotSupported otherwise.
+template <typename VT>
+cudaError_t launch_cluster_run(RunParams &p, const void *vals, cudaStream_t stream) {
+  const int spc = (p.nslices + kClusterCtas - 1) / kClusterCtas;
+  if (spc > kClusterSlices * kRunWarps) return cudaErrorNotSupported;
+  const size_t smem = sizeof(double) * cluster_run_doubles(spc, p.m);
+  // device limits, once per device: dynamic shared memory and whether a 16-CTA cluster of that size exists
+  static std::atomic<int> most[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorNotSupported;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kClusterCtas);
+  cfg.blockDim = dim3(kRunThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kClusterCtas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  int limit = most[dev].load(std::memory_order_acquire);
+  if (limit == 0) {
+    limit = -1;
+    cudaFuncAttributes fa;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(gs_cluster_run_kernel<VT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        allow_max_dynamic_smem(gs_cluster_run_kernel<VT>) == cudaSuccess &&
+        cudaFuncGetAttributes(&fa, gs_cluster_run_kernel<VT>) == cudaSuccess) {
+      cfg.dynamicSmemBytes = (size_t)fa.maxDynamicSharedSizeBytes;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&clusters, gs_cluster_run_kernel<VT>, &cfg) == cudaSuccess && clusters > 0)
+        limit = fa.maxDynamicSharedSizeBytes;
+    }
+    cudaGetLastError();
+    most[dev].store(limit, std::memory_order_release);
+  }
+  if (limit < 0 || smem > (size_t)limit) return cudaErrorNotSupported;
+  p.spc = spc;
+  cfg.dynamicSmemBytes = smem;
+  cfg.numAttrs = 2;
+  e = cudaLaunchKernelEx(&cfg, gs_cluster_run_kernel<VT>, p, static_cast<const VT *>(vals));
+  count_launch();
+  return e;
 }
 
 __global__ void gs_reset_kernel(GsState *st) {
@@ -572,6 +1179,41 @@ cudaError_t gs_state_reset(const GsWork &w, cudaStream_t stream) {
 cudaError_t gs_orthogonalize_launch(const GsPassArgs &a, const GsWork &w, double eta, bool fresh,
                                     cudaStream_t stream) {
   return launch_column(a, w, eta, fresh ? 1 : 0, 0, stream);
+}
+
+cudaError_t gs_run_launch(const GsRunArgs &a, const SpmvSell &S, bool f32, const GsWork &w, double eta,
+                          unsigned long long epoch, cudaStream_t stream) {
+  if (!w.slots || S.nrest > 0 || S.nslices <= 0 || a.m >= kMaxCols) return cudaErrorNotSupported;
+  RunParams p;
+  p.V = a.V;
+  p.ld = a.ld;
+  p.n = a.n;
+  p.k = a.k;
+  p.m = a.m;
+  p.coefbuf = a.coefbuf;
+  p.ldc = a.ldc;
+  p.T = a.T;
+  p.ldt = a.ldt;
+  p.st = w.st;
+  p.slots = w.slots;
+  p.epoch = epoch;
+  p.eta = eta;
+  p.deftol = kDefTol;
+  p.nslices = S.nslices;
+  p.off = S.off;
+  p.width = S.width;
+  p.cols = S.cols;
+  cudaError_t e = f32 ? launch_cluster_run<float>(p, S.vals, stream) : launch_cluster_run<double>(p, S.vals, stream);
+  if (e != cudaErrorNotSupported) return e;
+  const int ctas = w.num_sms < w.max_ctas ? w.num_sms : w.max_ctas;
+  const int spc = (S.nslices + ctas - 1) / ctas;
+  if (spc > kRunWarps) return cudaErrorNotSupported;
+  const int R = 32 * spc, parts = kRunWarps / spc;
+  const size_t smem = sizeof(double) * (size_t)R * (1 + parts + a.m + 1);
+  if (smem > kRunSmem) return cudaErrorNotSupported;
+  p.spc = spc;
+  const int G = (S.nslices + spc - 1) / spc;
+  return f32 ? launch_run<float>(p, S.vals, G, smem, stream) : launch_run<double>(p, S.vals, G, smem, stream);
 }
 
 cudaError_t gs_record_launch(const GsWork &w, double *out, cudaStream_t stream) {

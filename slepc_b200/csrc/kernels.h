@@ -129,6 +129,7 @@ struct GsWork {
   GsState *st;        // control block
   double *cnew;       // [kMaxCols+1] result of the last plain dot
   double *partials;   // [2 * (kMaxCols+1) * max_ctas] per-CTA partial dots of two passes
+  ulonglong2 *slots;  // [2 * (columns + 1) * max_ctas] exchange slots of whole-run launches (null: none)
   int max_ctas;
   int num_sms;
 };
@@ -151,6 +152,21 @@ struct GsPassArgs {
 // cooperative launch).  fresh: the column starts a run (or stands alone), so the control block's
 // counters and halt flag start from it.
 cudaError_t gs_orthogonalize_launch(const GsPassArgs &a, const GsWork &w, double eta, bool fresh, cudaStream_t stream);
+// A whole Lanczos run (columns k+1..m of V from column k) in one cooperative launch, when the rows of the
+// run's basis fit the shared memory of the chip and every row of the operator is in the slices of S;
+// cudaErrorNotSupported otherwise.  Fills coefbuf, T and the control block as the column-by-column run does.
+struct GsRunArgs {
+  double *V;
+  int ld, n, k, m;
+  double *coefbuf;
+  int ldc;
+  double *T;
+  int ldt;
+};
+// epoch: a number no earlier run on w.slots has used an epoch above; a run uses at most kRunEpochs per column.
+constexpr int kRunEpochs = 8;
+cudaError_t gs_run_launch(const GsRunArgs &a, const SpmvSell &S, bool f32, const GsWork &w, double eta,
+                          unsigned long long epoch, cudaStream_t stream);
 // Clear the control block (at creation, and after an error has been read back).
 cudaError_t gs_state_reset(const GsWork &w, cudaStream_t stream);
 // out[0..2] = norm, lindep flag and error bits of the last orthogonalisation (no host sync).

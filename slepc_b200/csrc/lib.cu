@@ -665,6 +665,7 @@ static void bv_free(b200_bv bv) {
   dev_free(bv->gs.st);
   dev_free(bv->gs.cnew);
   dev_free(bv->gs.partials);
+  dev_free(bv->gs.slots);
   dev_free(bv->coefbuf);
   dev_free(bv->hvec);
   dev_free(bv->T);
@@ -735,6 +736,8 @@ extern "C" b200_status b200_bv_create(int n, int m, void *stream, b200_bv *out) 
   ok = ok && dev_malloc(&bv->gs.st, sizeof(GsState)) == cudaSuccess;
   ok = ok && dev_malloc(&bv->gs.cnew, sizeof(double) * (kMaxCols + 1)) == cudaSuccess;
   ok = ok && dev_malloc(&bv->gs.partials, sizeof(double) * (size_t)(kMaxCols + 1) * 2 * sms) == cudaSuccess;
+  const size_t slot_bytes = sizeof(ulonglong2) * 2 * (size_t)(m + 2) * sms;
+  ok = ok && dev_malloc(&bv->gs.slots, slot_bytes) == cudaSuccess;
   ok = ok && dev_malloc(&bv->coefbuf, sizeof(double) * (size_t)bv->ldc * (m + 1)) == cudaSuccess;
   ok = ok && dev_malloc(&bv->hvec, sizeof(double) * (kMaxCols + 1)) == cudaSuccess;
   ok = ok && dev_malloc(&bv->T, sizeof(double) * 2 * (size_t)bv->ldt) == cudaSuccess;
@@ -749,6 +752,7 @@ extern "C" b200_status b200_bv_create(int n, int m, void *stream, b200_bv *out) 
   }
   cudaError_t e = cudaMemsetAsync(bv->V, 0, sizeof(double) * ((size_t)bv->ld * (m + 1) + 32), bv->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(bv->coefbuf, 0, sizeof(double) * (size_t)bv->ldc * (m + 1), bv->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(bv->gs.slots, 0, slot_bytes, bv->stream);  // epoch 0: never used
   if (e == cudaSuccess) e = gs_state_reset(bv->gs, bv->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(bv->stream);
   if (e != cudaSuccess) {
@@ -1591,7 +1595,15 @@ static b200_status bv_lanczos(b200_bv bv, b200_mat A, int k, int *m, double *alp
     timer->reserve((size_t)4 * (m0 - k) + 4);
     timer->used = 0;
   }
-  for (int j = k; j < m0; ++j) {
+  // one launch for the whole run where the basis fits the chip; timing needs the kernels one by one
+  cudaError_t whole = cudaErrorNotSupported;
+  if (!timing && A->kind == kMatCsr && A->schedule == B200_SPMV_SELL && A->a.sell_ready) {
+    const GsRunArgs r{bv->V, bv->ld, bv->n, k, m0, bv->coefbuf, bv->ldc, bv->T, bv->ldt};
+    whole = gs_run_launch(r, A->a.sell, A->a.f32, bv->gs, bv->eta, bv->run_epoch, bv->stream);
+    if (whole != cudaErrorNotSupported) B200_CUDA_CHECK(whole);
+    if (whole == cudaSuccess) bv->run_epoch += (unsigned long long)kRunEpochs * (m0 - k);
+  }
+  for (int j = k; j < m0 && whole == cudaErrorNotSupported; ++j) {
     cudaEvent_t e0 = timing ? timer->next() : nullptr, e1 = timing ? timer->next() : nullptr;
     cudaEvent_t e2 = timing ? timer->next() : nullptr, e3 = timing ? timer->next() : nullptr;
     if (e0) cudaEventRecord(e0, bv->stream);

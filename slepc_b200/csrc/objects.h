@@ -56,6 +56,7 @@ struct b200_bv_s {
   int orthog_block = B200_ORTHOG_BLOCK_GS;  // bvfunc.c:179
   cudaStream_t stream = nullptr;
   b200::GsWork gs{};
+  unsigned long long run_epoch = 0;  // epochs used so far on gs.slots
   double *coefbuf = nullptr;  // (m+1) x (m+1): column j = coefficients of column j (BVGetBufferVec)
   int ldc = 0;
   double *hvec = nullptr;     // coefficients of the vector variant
