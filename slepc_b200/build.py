@@ -57,7 +57,7 @@ def build_generator(force=False):
 
 def build(force=False, verbose=False):
     os.makedirs(BUILD, exist_ok=True)
-    headers = glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    headers = glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
     objs = []
     for src in sources():
         obj = os.path.join(BUILD, os.path.basename(src) + ".o")

@@ -31,6 +31,7 @@
 
 #include "common.h"
 #include "kernels.h"
+#include "neural_fused.cuh"
 
 struct b200_neural_op_s {
   int N = 0, P = 0, W = 0, M = 0, L = 0, H = 0, K = 0;
@@ -48,7 +49,14 @@ struct b200_neural_op_s {
   float *act = nullptr;
   size_t act_len = 0;
   float *loss_bk = nullptr;  // B x K per-output losses
-  std::vector<float> hloss;
+  bool fused = false;        // the one-pass kernels of neural_fused.cuh serve these sizes
+  float *Sp = nullptr;       // sine basis padded to neural::kModes columns
+  float *bias_part = nullptr;      // blocks' partial sums of the bias gradients
+  float *mode_work = nullptr;      // modes_kernel: the blocks' shares and arrival counts
+  unsigned *mode_count = nullptr;
+  float2 *loss_part = nullptr, *loss_coef = nullptr;
+  float *hloss = nullptr;    // pinned: B x K losses, then the error word
+  cudaEvent_t loss_ready = nullptr;
   float *ws = nullptr;       // split-depth partial products of the GEMMs
   size_t ws_len = 0;
   int *dev_err = nullptr;    // device error bits of the GEMMs (bounded waits)
@@ -62,10 +70,8 @@ struct MView {
   long long rs, cs, bs;  // element (i, j) of matrix z at p + z*bs + i*rs + j*cs
 };
 
-__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-  return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
-}
+using neural::gelu;
+using neural::gelu_grad;
 
 // U[b][c][p] += bias[c]; V = act ? gelu(U) : U
 __global__ void bias_act_kernel(float *U, const float *__restrict__ bias, float *V, int C, int P, long long total,
@@ -212,23 +218,51 @@ Acts carve(b200_neural_op op, size_t *len) {
   return a;
 }
 
+// Blocks of a field in modes_kernel.
+int mode_blocks(b200_neural_op op) { return (op->N + neural::kModeCols - 1) / neural::kModeCols; }
+// Partial bias-gradient sums: rows (channels of every bias) and blocks of points per row.
+int bias_rows(b200_neural_op op) { return op->W * (op->L + 1) + op->H + op->K; }
+long long bias_blocks(b200_neural_op op, int B) {
+  return (long long)B * ((op->P + neural::kTile - 1) / neural::kTile);
+}
+
 b200_status reserve(b200_neural_op op, int B) {
   if (B <= op->cap && op->act) return B200_OK;
   cudaFree(op->act);
   cudaFree(op->loss_bk);
+  cudaFree(op->bias_part);
+  cudaFree(op->loss_part);
+  cudaFree(op->mode_work);
+  cudaFree(op->mode_count);
+  cudaFreeHost(op->hloss);
   op->act = nullptr;
   op->loss_bk = nullptr;
+  op->bias_part = op->mode_work = nullptr;
+  op->mode_count = nullptr;
+  op->loss_part = op->loss_coef = nullptr;
+  op->hloss = nullptr;
   op->cap = B;
   size_t len = 0;
   carve(op, &len);
-  if (cudaMalloc(&op->act, sizeof(float) * len) != cudaSuccess ||
-      cudaMalloc(&op->loss_bk, sizeof(float) * (size_t)B * op->K) != cudaSuccess) {
+  const size_t BK = (size_t)B * op->K, slices = ((size_t)op->P + neural::kLossSlice - 1) / neural::kLossSlice;
+  bool ok = cudaMalloc(&op->act, sizeof(float) * len) == cudaSuccess &&
+            cudaMalloc(&op->loss_bk, sizeof(float) * BK) == cudaSuccess &&
+            cudaMallocHost(&op->hloss, sizeof(float) * BK + sizeof(int)) == cudaSuccess;
+  if (ok && op->fused)
+    ok = cudaMalloc(&op->bias_part, sizeof(float) * (size_t)bias_rows(op) * bias_blocks(op, B)) == cudaSuccess &&
+         cudaMalloc(&op->mode_work, sizeof(float) * (size_t)B * op->W * mode_blocks(op) * neural::kModeThreads) ==
+             cudaSuccess &&
+         cudaMalloc(&op->mode_count, sizeof(unsigned) * (size_t)B * op->W) == cudaSuccess &&
+         cudaMemsetAsync(op->mode_count, 0, sizeof(unsigned) * (size_t)B * op->W, op->stream) == cudaSuccess &&
+         cudaMalloc(&op->loss_part, sizeof(float2) * BK * (slices + 1)) == cudaSuccess;
+  if (!ok) {
     cudaFree(op->act);
     op->act = nullptr;
     op->cap = 0;
     b200_set_last_error(__FILE__, __LINE__, "cudaMalloc failed for the neural-operator activations");
     return B200_ERR_NOMEM;
   }
+  if (op->fused) op->loss_coef = op->loss_part + BK * slices;
   op->act_len = len;
   // split-depth workspace: the widest summed weight gradient over the batch, four depth splits
   const size_t W = op->W, mn = std::max({W * 3, W * W, (size_t)op->H * W, (size_t)op->K * op->H});
@@ -383,20 +417,170 @@ b200_status backward(b200_neural_op op, int B, Acts &a) {
   return B200_OK;
 }
 
-b200_status loss(b200_neural_op op, int B, const float *targets, Acts &a, bool want_grad, float *loss_out) {
+// The loss of every output is on its way to the host (with the error word) when loss_read is called: the
+// host waits for that copy alone, not for a backward pass queued behind it.
+b200_status loss_queue_read(b200_neural_op op, int B) {
+  const size_t n = (size_t)B * op->K;
+  B200_CUDA_CHECK(cudaMemcpyAsync(op->hloss, op->loss_bk, sizeof(float) * n, cudaMemcpyDeviceToHost, op->stream));
+  B200_CUDA_CHECK(cudaMemcpyAsync(op->hloss + n, op->dev_err, sizeof(int), cudaMemcpyDeviceToHost, op->stream));
+  B200_CUDA_CHECK(cudaEventRecord(op->loss_ready, op->stream));
+  return B200_OK;
+}
+b200_status loss_read(b200_neural_op op, int B, float *loss_out) {
+  B200_CUDA_CHECK(cudaEventSynchronize(op->loss_ready));
+  const size_t n = (size_t)B * op->K;
+  int e = 0;
+  memcpy(&e, op->hloss + n, sizeof(int));
+  if (e) return gemm_status(op);
+  double s = 0.0;
+  for (size_t i = 0; i < n; ++i) s += op->hloss[i];
+  if (loss_out) *loss_out = (float)(s / (double)n);
+  return B200_OK;
+}
+
+b200_status loss(b200_neural_op op, int B, const float *targets, Acts &a, bool want_grad) {
   const float scale = 1.f / (float)(B * op->K);
   loss_kernel<<<dim3(op->K, B), 256, 0, op->stream>>>(a.Y, targets, op->K, op->P, scale, op->loss_bk,
                                                       want_grad ? a.dY : nullptr);
   count_launch();
   B200_CUDA_CHECK(cudaGetLastError());
-  op->hloss.resize((size_t)B * op->K);
-  B200_CUDA_CHECK(cudaMemcpyAsync(op->hloss.data(), op->loss_bk, sizeof(float) * op->hloss.size(),
-                                  cudaMemcpyDeviceToHost, op->stream));
-  B200_CUDA_CHECK(cudaStreamSynchronize(op->stream));
-  B200_CHECK(gemm_status(op));
-  double s = 0.0;
-  for (float v : op->hloss) s += v;
-  if (loss_out) *loss_out = (float)(s / (double)op->hloss.size());
+  return loss_queue_read(op, B);
+}
+
+// ---- the one-pass form (neural_fused.cuh)
+
+cudaError_t pw(b200_neural_op op, int B, const neural::PwArgs &a) {
+  const int rows = a.T2 ? (neural::kTile - 1) / op->N + 2 : 0;
+  const size_t smem = sizeof(float) * ((size_t)neural::kTile * (std::max(a.Ci, 32) + (a.Ug ? 32 : 0)) +
+                                       32 * ((size_t)a.Ci + (size_t)rows * neural::kModes));
+  const dim3 grid((op->P + neural::kTile - 1) / neural::kTile, B, (a.Co + 31) / 32);
+  neural::pw_kernel<<<grid, neural::kPwThreads, smem, op->stream>>>(a);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t field_modes(b200_neural_op op, int nz, const float *X, float *C) {
+  neural::modes_kernel<<<dim3(nz, mode_blocks(op)), neural::kModeThreads, neural::kModeSmem, op->stream>>>(
+      X, op->Sp, op->N, op->M, C, op->mode_work, op->mode_count);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t mode_mix(b200_neural_op op, int B, const float *R, const float *in, float *T2, int transposed,
+                     const float *C, float *dR) {
+  neural::mode_mix_kernel<<<op->W * B + (dR ? op->W * op->W : 0), 256, 0, op->stream>>>(R, in, op->Sp, T2, B, op->W, op->N,
+                                                                                       op->M, transposed, C, dR);
+  count_launch();
+  return cudaGetLastError();
+}
+
+b200_status forward_fused(b200_neural_op op, int B, const float *feat, Acts &a, float *Y) {
+  const int W = op->W, L = op->L, M = op->M, H = op->H, K = op->K;
+  const size_t WP = (size_t)W * op->P, M2 = (size_t)M * M;
+  neural::PwArgs g{};
+  g.N = op->N;
+  g.P = op->P;
+  g.M = M;
+  g.Sp = op->Sp;
+  g.X = feat;
+  g.Ci = 3;
+  g.Co = W;
+  g.Wt = prm(op, op->oPw);
+  g.wo = 3;
+  g.wc = 1;
+  g.bias = prm(op, op->oPb);
+  g.V = a.V;
+  B200_CUDA_CHECK(pw(op, B, g));
+  g.Ci = W;
+  g.wo = W;
+  for (int l = 0; l < L; ++l) {
+    float *Vl = a.V + l * B * WP, *Cl = a.Ch + l * B * W * M2;
+    B200_CUDA_CHECK(field_modes(op, B * W, Vl, Cl));
+    B200_CUDA_CHECK(mode_mix(op, B, prm(op, op->oR[l]), Cl, a.T2, 0, nullptr, nullptr));
+    g.X = Vl;
+    g.Wt = prm(op, op->oW[l]);
+    g.T2 = a.T2;
+    g.bias = prm(op, op->ob[l]);
+    g.act = l < L - 1;
+    g.U = g.act ? a.U + l * B * WP : nullptr;
+    g.V = a.V + (l + 1) * B * WP;
+    B200_CUDA_CHECK(pw(op, B, g));
+  }
+  const int Hp = (H + 31) & ~31;
+  const size_t smem = sizeof(float) * ((size_t)(W + 32) * neural::kTile + (size_t)W * Hp + (size_t)Hp * 16 + Hp);
+  neural::proj_fwd_kernel<<<dim3((op->P + neural::kTile - 1) / neural::kTile, B), neural::kPwThreads, smem, op->stream>>>(
+      a.V + L * B * WP, W, H, K, op->P, prm(op, op->oQ1), prm(op, op->oq1), prm(op, op->oQ2), prm(op, op->oq2), a.Z, a.Hh, Y);
+  count_launch();
+  B200_CUDA_CHECK(cudaGetLastError());
+  return B200_OK;
+}
+
+b200_status loss_fused(b200_neural_op op, int B, const float *targets, const float *Y) {
+  const int slices = (op->P + neural::kLossSlice - 1) / neural::kLossSlice, BK = B * op->K;
+  neural::loss_part_kernel<<<dim3(slices, op->K, B), 256, 0, op->stream>>>(Y, targets, op->K, op->P, op->loss_part);
+  count_launch();
+  neural::loss_final_kernel<<<(BK + 127) / 128, 128, 0, op->stream>>>(op->loss_part, slices, BK, 1.f / (float)BK, op->loss_bk,
+                                                                     op->loss_coef);
+  count_launch();
+  B200_CUDA_CHECK(cudaGetLastError());
+  return loss_queue_read(op, B);
+}
+
+b200_status backward_fused(b200_neural_op op, int B, const float *feat, const float *targets, Acts &a) {
+  const int W = op->W, L = op->L, M = op->M, H = op->H, K = op->K;
+  const size_t WP = (size_t)W * op->P, M2 = (size_t)M * M;
+  // partial bias sums, tensor by tensor: rows of this tensor's blocks
+  neural::BiasRows br{};
+  int rows = 0;
+  long long at = 0;
+  auto bias = [&](int channels, size_t off) {
+    const int t = br.count++;
+    br.first[t] = rows;
+    br.blocks[t] = (int)bias_blocks(op, B);
+    br.at[t] = at;
+    br.off[t] = (long long)off;
+    rows += channels;
+    at += (long long)channels * br.blocks[t];
+    return op->bias_part + br.at[t];
+  };
+  float *part_k = bias(K, op->oq2), *part_h = bias(H, op->oq1), *part_w = bias(W, op->ob[L - 1]);
+  const int Hp = (H + 31) & ~31;
+  const size_t smem = sizeof(float) * ((size_t)(64 + K) * neural::kTile + (size_t)K * Hp + (size_t)Hp * 32);
+  float *dU = a.dV0, *next = a.dV1;  // dU holds the gradient before layer l's activation
+  neural::proj_bwd_kernel<<<dim3((op->P + neural::kTile - 1) / neural::kTile, B, (W + 31) / 32),
+                                neural::kPwThreads, smem, op->stream>>>(
+      a.Y, targets, op->loss_coef, a.Z, W, H, K, op->P, prm(op, op->oQ1), prm(op, op->oQ2), a.dY, a.dH, dU, part_k, part_h,
+      part_w);
+  count_launch();
+  B200_CUDA_CHECK(cudaGetLastError());
+  B200_CUDA_CHECK(mix_grad(op, B, K, H, a.dY, a.Hh, grd(op, op->oQ2)));
+  B200_CUDA_CHECK(mix_grad(op, B, H, W, a.dH, a.V + L * B * WP, grd(op, op->oQ1)));
+  neural::PwArgs g{};
+  g.Ci = W;
+  g.Co = W;
+  g.N = op->N;
+  g.P = op->P;
+  g.M = M;
+  g.Sp = op->Sp;
+  g.wo = 1;  // W_l^T
+  g.wc = W;
+  g.T2 = a.T2;
+  for (int l = L - 1; l >= 0; --l) {
+    B200_CUDA_CHECK(mix_grad(op, B, W, W, dU, a.V + l * B * WP, grd(op, op->oW[l])));
+    B200_CUDA_CHECK(field_modes(op, B * W, dU, a.dDh));
+    B200_CUDA_CHECK(mode_mix(op, B, prm(op, op->oR[l]), a.dDh, a.T2, 1, a.Ch + l * B * W * M2, grd(op, op->oR[l])));
+    g.X = dU;
+    g.Wt = prm(op, op->oW[l]);
+    g.Ug = l > 0 ? a.U + (l - 1) * B * WP : nullptr;
+    g.V = next;
+    g.part = bias(W, l > 0 ? op->ob[l - 1] : op->oPb);
+    B200_CUDA_CHECK(pw(op, B, g));
+    std::swap(dU, next);
+  }
+  B200_CUDA_CHECK(mix_grad(op, B, W, 3, dU, feat, grd(op, op->oPw)));
+  neural::bias_rows_kernel<<<rows, 128, 0, op->stream>>>(op->bias_part, br, op->grads);
+  count_launch();
+  B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
 
@@ -437,7 +621,16 @@ extern "C" b200_status b200_neural_op_create(int N, int width, int modes, int la
   op->oQ2 = take((size_t)nout * hidden);
   op->oq2 = take(nout);
   op->nparams = off;
-  bool ok = cudaMalloc(&op->params, sizeof(float) * off) == cudaSuccess &&
+  // the one-pass kernels: channel counts and modes that fit their registers and shared memory, and rows long
+  // enough that a block of points touches few of them; other networks go through separate products
+  op->fused = W <= 64 && modes <= neural::kModes && hidden <= 128 && nout <= 16 && N >= 32;
+  bool ok = cudaEventCreateWithFlags(&op->loss_ready, cudaEventDisableTiming) == cudaSuccess &&
+            cudaMalloc(&op->Sp, sizeof(float) * (size_t)N * neural::kModes) == cudaSuccess &&
+            (!op->fused || (allow_max_dynamic_smem(neural::pw_kernel) == cudaSuccess &&
+                            allow_max_dynamic_smem(neural::modes_kernel) == cudaSuccess &&
+                            allow_max_dynamic_smem(neural::proj_fwd_kernel) == cudaSuccess &&
+                            allow_max_dynamic_smem(neural::proj_bwd_kernel) == cudaSuccess)) &&
+            cudaMalloc(&op->params, sizeof(float) * off) == cudaSuccess &&
             cudaMalloc(&op->grads, sizeof(float) * off) == cudaSuccess &&
             cudaMalloc(&op->adam_m, sizeof(float) * off) == cudaSuccess &&
             cudaMalloc(&op->adam_v, sizeof(float) * off) == cudaSuccess &&
@@ -448,7 +641,11 @@ extern "C" b200_status b200_neural_op_create(int N, int width, int modes, int la
     const double c = std::sqrt(2.0 / (N + 1));
     for (int i = 0; i < N; ++i)
       for (int k = 0; k < modes; ++k) S[(size_t)i * modes + k] = (float)(c * std::sin(M_PI * (i + 1) * (k + 1) / (N + 1)));
-    ok = cudaMemcpyAsync(op->S, S.data(), sizeof(float) * S.size(), cudaMemcpyHostToDevice, op->stream) == cudaSuccess &&
+    std::vector<float> Sp((size_t)N * neural::kModes, 0.f);
+    for (int i = 0; i < N; ++i)
+      for (int k = 0; k < std::min(modes, neural::kModes); ++k) Sp[(size_t)i * neural::kModes + k] = S[(size_t)i * modes + k];
+    ok = cudaMemcpyAsync(op->Sp, Sp.data(), sizeof(float) * Sp.size(), cudaMemcpyHostToDevice, op->stream) == cudaSuccess &&
+         cudaMemcpyAsync(op->S, S.data(), sizeof(float) * S.size(), cudaMemcpyHostToDevice, op->stream) == cudaSuccess &&
          cudaMemsetAsync(op->params, 0, sizeof(float) * off, op->stream) == cudaSuccess &&
          cudaMemsetAsync(op->adam_m, 0, sizeof(float) * off, op->stream) == cudaSuccess &&
          cudaMemsetAsync(op->adam_v, 0, sizeof(float) * off, op->stream) == cudaSuccess &&
@@ -471,8 +668,15 @@ extern "C" b200_status b200_neural_op_destroy(b200_neural_op op) {
   cudaFree(op->adam_m);
   cudaFree(op->adam_v);
   cudaFree(op->S);
+  cudaFree(op->Sp);
   cudaFree(op->act);
   cudaFree(op->loss_bk);
+  cudaFree(op->bias_part);
+  cudaFree(op->loss_part);
+  cudaFree(op->mode_work);
+  cudaFree(op->mode_count);
+  cudaFreeHost(op->hloss);
+  if (op->loss_ready) cudaEventDestroy(op->loss_ready);
   cudaFree(op->ws);
   cudaFree(op->dev_err);
   delete op;
@@ -507,9 +711,13 @@ extern "C" b200_status b200_neural_op_forward(b200_neural_op op, int batch, cons
   B200_CHECK(reserve(op, batch));
   size_t len;
   Acts a = carve(op, &len);
-  B200_CHECK(forward(op, batch, features_dev, a));
-  B200_CUDA_CHECK(cudaMemcpyAsync(out_dev, a.Y, sizeof(float) * (size_t)batch * op->K * op->P,
-                                  cudaMemcpyDeviceToDevice, op->stream));
+  if (op->fused) {
+    B200_CHECK(forward_fused(op, batch, features_dev, a, out_dev));
+  } else {
+    B200_CHECK(forward(op, batch, features_dev, a));
+    B200_CUDA_CHECK(cudaMemcpyAsync(out_dev, a.Y, sizeof(float) * (size_t)batch * op->K * op->P,
+                                    cudaMemcpyDeviceToDevice, op->stream));
+  }
   B200_CUDA_CHECK(cudaStreamSynchronize(op->stream));
   return gemm_status(op);
 }
@@ -520,9 +728,16 @@ extern "C" b200_status b200_neural_op_loss_grad(b200_neural_op op, int batch, co
   B200_CHECK(reserve(op, batch));
   size_t len;
   Acts a = carve(op, &len);
-  B200_CHECK(forward(op, batch, features_dev, a));
-  B200_CHECK(loss(op, batch, targets_dev, a, true, loss_out));
-  B200_CHECK(backward(op, batch, a));
+  if (op->fused) {
+    B200_CHECK(forward_fused(op, batch, features_dev, a, a.Y));
+    B200_CHECK(loss_fused(op, batch, targets_dev, a.Y));
+    B200_CHECK(backward_fused(op, batch, features_dev, targets_dev, a));
+  } else {
+    B200_CHECK(forward(op, batch, features_dev, a));
+    B200_CHECK(loss(op, batch, targets_dev, a, true));
+    B200_CHECK(backward(op, batch, a));
+  }
+  B200_CHECK(loss_read(op, batch, loss_out));
   if (grads_host) {
     B200_CUDA_CHECK(
         cudaMemcpyAsync(grads_host, op->grads, sizeof(float) * op->nparams, cudaMemcpyDeviceToHost, op->stream));
@@ -552,6 +767,12 @@ extern "C" b200_status b200_neural_op_loss(b200_neural_op op, int batch, const f
   B200_CHECK(reserve(op, batch));
   size_t len;
   Acts a = carve(op, &len);
-  B200_CHECK(forward(op, batch, features_dev, a));
-  return loss(op, batch, targets_dev, a, false, loss_out);
+  if (op->fused) {
+    B200_CHECK(forward_fused(op, batch, features_dev, a, a.Y));
+    B200_CHECK(loss_fused(op, batch, targets_dev, a.Y));
+  } else {
+    B200_CHECK(forward(op, batch, features_dev, a));
+    B200_CHECK(loss(op, batch, targets_dev, a, false));
+  }
+  return loss_read(op, batch, loss_out);
 }

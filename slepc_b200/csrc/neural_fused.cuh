@@ -1,0 +1,681 @@
+// Fused kernels of the neural operator (learned.cu) for networks of ordinary width.
+//
+// A pointwise step of the network is a contraction over at most 64 channels plus 16 modes per grid point:
+// 4 FP32 multiply-adds per byte that must move, so HBM bounds it and not the arithmetic.  These kernels
+// therefore do each step in one pass over the activations: channel mix, spectral term, bias, activation
+// (or its derivative) and the bias gradients' partial sums, in FP32 FMAs (packed two to an instruction,
+// fma.rn.f32x2) with the weights broadcast from shared memory.  The weight gradients, whose contraction
+// runs over the grid, stay tensor-core products (tcgemm.cu).
+//
+// Measured (loss and gradients, width 32, 16 modes, 4 layers): 512 x 512 grid, batch 4, 12.2 ms as separate
+// products and elementwise kernels (113 launches), 4.4 ms so (44 launches); 64 x 64 grid, batch 16, 1.55 -> 0.96 ms.
+#pragma once
+#include "common.h"
+
+namespace b200 {
+namespace neural {
+
+constexpr int kTile = 256;       // grid points per block
+constexpr int kPwThreads = 128;  // two halves of 64 threads: a thread has 4 points (64 apart) and its half's 16 outputs
+constexpr int kModes = 16;       // modes per direction, zero-padded
+
+__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
+__device__ __forceinline__ float gelu_grad(float x) {
+  return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
+}
+
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+// The 4 points x 16 outputs of a thread, outputs in pairs.
+struct Acc {
+  unsigned long long v[4][8];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int o = 0; o < 8; ++o) v[u][o] = 0ull;
+  }
+  __device__ __forceinline__ float get(int u, int o) const {
+    const float2 f = unpack2(v[u][o >> 1]);
+    return o & 1 ? f.y : f.x;
+  }
+};
+// acc(u, o) += w[o] x[u]; w 16-byte aligned shared memory, the same for every lane.  A uniform 16-byte shared
+// load takes the port as long as four of 4 bytes, so 4 points share each: 20 cycles of the port per channel
+// and warp for 64 multiply-adds a lane (34 with 2 points and 32 outputs, which bounded pw_kernel at 245 us).
+__device__ __forceinline__ void axpy4(Acc &acc, const float *w, const float (&x)[4]) {
+  ulonglong2 ww[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) ww[q] = reinterpret_cast<const ulonglong2 *>(w)[q];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const unsigned long long xx = pack2(x[u], x[u]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      fma2(acc.v[u][2 * q], ww[q].x, xx);
+      fma2(acc.v[u][2 * q + 1], ww[q].y, xx);
+    }
+  }
+}
+// acc += W^T X over `channels` rows of the staged tile X ([channel][kTile]) with weights [channel][ldw]
+__device__ __forceinline__ void mix16(Acc &acc, const float *X, const float *W, int ldw, int channels, int t) {
+#pragma unroll 2
+  for (int c = 0; c < channels; ++c) {
+    float x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = X[c * kTile + t + 64 * u];
+    axpy4(acc, W + c * ldw, x);
+  }
+}
+
+// the 4 points x 16 outputs of a thread to its rows of a [16][kTile] tile
+__device__ __forceinline__ void acc_to_tile(const Acc &acc, float *tile, int t) {
+#pragma unroll
+  for (int o = 0; o < 16; o += 2)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float2 f = unpack2(acc.v[u][o >> 1]);
+      tile[o * kTile + t + 64 * u] = f.x;
+      tile[(o + 1) * kTile + t + 64 * u] = f.y;
+    }
+}
+
+// Partial sums of a bias gradient over the block's points from the tile R ([channel][kTile]): part[c * stride]
+// gets channel c < nc (the blocks' sums are added in order afterwards).
+__device__ __forceinline__ void tile_sums(const float *R, int nc, float *part, size_t stride) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncthreads();
+  for (int c = warp; c < nc; c += kPwThreads / 32) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < kTile / 32; ++q) s += R[c * kTile + lane + 32 * q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) part[c * stride] = s;
+  }
+}
+
+// Stage `channels` rows of `width` points (from point p0 of fields of P points; zeros past P) in shared memory
+// with asynchronous copies, so that a block has its whole tile in flight at once (plain loads in the channel
+// loop left 12 KB in flight per SM, and pw_kernel at 360 us where 90 are due to its bytes): 16 bytes each when
+// the fields allow it, 4 otherwise.
+template <int WIDTH>
+__device__ __forceinline__ void stage_tile(float *dst, const float *src, int channels, int P, int p0) {
+  const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(dst);
+  if ((P & 3) == 0 && ((uintptr_t)src & 15) == 0 && p0 + WIDTH <= P) {
+    for (int e = threadIdx.x; e < channels * (WIDTH / 4); e += kPwThreads) {
+      const int c = e / (WIDTH / 4), q = e % (WIDTH / 4);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d0 + 16u * (uint32_t)e),
+                   "l"(src + (size_t)c * P + p0 + 4 * q)
+                   : "memory");
+    }
+  } else {
+    for (int e = threadIdx.x; e < channels * WIDTH; e += kPwThreads) {
+      const int c = e / WIDTH, q = e % WIDTH;
+      const bool in = p0 + q < P;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d0 + 4u * (uint32_t)e),
+                   "l"(src + (in ? (size_t)c * P + p0 + q : 0)), "r"(in ? 4 : 0)
+                   : "memory");
+    }
+  }
+}
+__device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+struct PwArgs {
+  const float *X;        // input, batch x Ci x P
+  int Ci, Co, N, P;
+  const float *Wt;       // weight of (output o, input c) at o * wo + c * wc
+  int wo, wc;
+  const float *T2;       // spectral weights, batch x Co x N x M (null: no spectral term)
+  const float *Sp;       // N x kModes sine basis, zero past M
+  int M;
+  const float *bias;     // Co (null: none)
+  const float *Ug;       // multiply the result by gelu'(Ug) (null: no)
+  float *U;              // the result before the activation (null: not wanted)
+  float *V;              // the result, through gelu when act
+  int act;
+  float *part;           // partial bias-gradient sums of the result, [Co][blocks] (null: none)
+};
+
+// out(o, p) = sum_c Wt(o, c) X(c, p) + sum_m T2(o, i, m) S(j, m) + bias(o) at the grid points p = i N + j of
+// sample blockIdx.y, outputs [32 z, 32 (z+1)) for z = blockIdx.z.  The spectral term enters as M further inputs
+// S(j, m) whose weights belong to the point's image row.
+//
+// Bound: HBM, one read of X (and Ug), one write of U and V (512 x 512 grid, batch 4, width 32: 403 MB, 62 us), and
+// beside it the issue slots of erff.  Measured there: 170 us forward, 196 us with gelu' in the backward pass,
+// where the separate products and elementwise kernels of a layer took 740 us.
+__global__ void __launch_bounds__(kPwThreads) pw_kernel(PwArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  const int tid = threadIdx.x, t = tid & 63, half = tid >> 6;
+  const int b = blockIdx.y, o0 = blockIdx.z * 32, p0 = blockIdx.x * kTile, no = min(32, a.Co - o0);
+  float *Xs = sm;                                 // [max(Ci, 32)][kTile]: the input, then the result
+  float *Gs = Xs + max(a.Ci, 32) * kTile;         // [32][kTile], with Ug
+  float *W = Gs + (a.Ug ? 32 * kTile : 0);        // [Ci][32]
+  float *T2 = W + a.Ci * 32;                      // [row][kModes][32]
+  stage_tile<kTile>(Xs, a.X + (size_t)b * a.Ci * a.P, a.Ci, a.P, p0);
+  if (a.Ug) stage_tile<kTile>(Gs, a.Ug + ((size_t)b * a.Co + o0) * a.P, no, a.P, p0);
+  stage_commit();
+  for (int e = tid; e < a.Ci * 32; e += kPwThreads) {
+    // neighbouring threads take neighbouring weights
+    const int c = a.wc == 1 ? e % a.Ci : e >> 5, o = a.wc == 1 ? e / a.Ci : e & 31;
+    W[c * 32 + o] = o < no ? __ldg(a.Wt + (o0 + o) * a.wo + c * a.wc) : 0.f;
+  }
+  const int i0 = p0 / a.N, nrows = (min(p0 + kTile, a.P) - 1) / a.N - i0 + 1;
+  if (a.T2)
+    for (int e = tid; e < nrows * kModes * 32; e += kPwThreads) {
+      const int m = e & 15, r = (e >> 4) % nrows, o = (e >> 4) / nrows;
+      T2[(r * kModes + m) * 32 + o] =
+          o < no && m < a.M ? __ldg(a.T2 + ((size_t)(b * a.Co + o0 + o) * a.N + i0 + r) * a.M + m) : 0.f;
+    }
+  Acc acc;
+#pragma unroll
+  for (int o = 0; o < 16; o += 2) {
+    const int q = 16 * half + o;
+    const float b0 = a.bias && q < no ? __ldg(a.bias + o0 + q) : 0.f, b1 = a.bias && q + 1 < no ? __ldg(a.bias + o0 + q + 1) : 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc.v[u][o >> 1] = pack2(b0, b1);
+  }
+  stage_wait();
+  __syncthreads();
+  mix16(acc, Xs, W + 16 * half, 32, a.Ci, t);
+  if (a.T2) {
+    const float *s[4];
+    int row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int p = min(p0 + t + 64 * u, a.P - 1), i = p / a.N;
+      row[u] = i - i0;
+      s[u] = a.Sp + (size_t)(p - i * a.N) * kModes;
+    }
+    if (nrows == 1) {
+      for (int m = 0; m < a.M; m += 4) {
+        float4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = __ldg(reinterpret_cast<const float4 *>(s[u] + m));
+        const float x0[4] = {q[0].x, q[1].x, q[2].x, q[3].x}, x1[4] = {q[0].y, q[1].y, q[2].y, q[3].y};
+        const float x2[4] = {q[0].z, q[1].z, q[2].z, q[3].z}, x3[4] = {q[0].w, q[1].w, q[2].w, q[3].w};
+        axpy4(acc, T2 + m * 32 + 16 * half, x0);
+        axpy4(acc, T2 + (m + 1) * 32 + 16 * half, x1);
+        axpy4(acc, T2 + (m + 2) * 32 + 16 * half, x2);
+        axpy4(acc, T2 + (m + 3) * 32 + 16 * half, x3);
+      }
+    } else {  // points of several image rows: each its own weights
+      for (int m = 0; m < a.M; ++m)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(T2 + (row[u] * kModes + m) * 32 + 16 * half);
+          const float x = __ldg(s[u] + m);
+          const unsigned long long xx = pack2(x, x);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const ulonglong2 ww = w[q];
+            fma2(acc.v[u][2 * q], ww.x, xx);
+            fma2(acc.v[u][2 * q + 1], ww.y, xx);
+          }
+        }
+    }
+  }
+  // The activation runs in a rolled loop over the results in shared memory: unrolled over a thread's 64
+  // registers its code overflows the instruction cache (1.3 of 6 stall cycles per instruction).
+  __syncthreads();  // the staged input is consumed
+  float *R = Xs;    // [32][kTile]
+  acc_to_tile(acc, R + 16 * half * kTile, t);
+  float *mine = R + 16 * half * kTile + t;
+  const float *ug = Gs + 16 * half * kTile + t;
+  const size_t at0 = ((size_t)b * a.Co + o0 + 16 * half) * a.P + p0 + t;
+  const int mo = min(16, no - 16 * half);
+#pragma unroll 1
+  for (int o = 0; o < mo; ++o) {
+    const size_t at = at0 + (size_t)o * a.P;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = p0 + t + 64 * u < a.P;
+      float x = mine[o * kTile + 64 * u];
+      if (a.U && in) a.U[at + 64 * u] = x;
+      if (a.Ug) x *= gelu_grad(ug[o * kTile + 64 * u]);
+      if (a.act) x = gelu(x);
+      if (in) a.V[at + 64 * u] = x;
+      if (a.part) mine[o * kTile + 64 * u] = in ? x : 0.f;
+    }
+  }
+  if (a.part) {
+    const size_t blocks = (size_t)gridDim.x * gridDim.y;
+    tile_sums(R, no, a.part + (size_t)o0 * blocks + (size_t)b * gridDim.x + blockIdx.x, blocks);
+  }
+}
+
+// Projection, forward: Z = Q1 V + q1, H = gelu(Z), Y = Q2 H + q2 (at most 16 outputs), 32 hidden channels at a
+// time (16 per half of the block; the halves' shares of Y meet at the end): V is read once, Z, H and Y are
+// written once.
+__global__ void __launch_bounds__(kPwThreads) proj_fwd_kernel(const float *__restrict__ V, int W, int H, int K, int P,
+                                                              const float *__restrict__ Q1, const float *__restrict__ q1,
+                                                              const float *__restrict__ Q2, const float *__restrict__ q2,
+                                                              float *Z, float *Hh, float *Y) {
+  extern __shared__ __align__(16) float sm[];
+  const int Hp = (H + 31) & ~31;
+  float *Xs = sm;              // [W][kTile]
+  float *Hs = Xs + W * kTile;  // [32][kTile]: Z then H of the group; at the end the second half's share of Y
+  float *w1 = Hs + 32 * kTile; // [W][Hp]
+  float *w2 = w1 + W * Hp;     // [Hp][16]
+  float *b1 = w2 + Hp * 16;    // [Hp]
+  const int tid = threadIdx.x, t = tid & 63, half = tid >> 6, b = blockIdx.y, p0 = blockIdx.x * kTile;
+  stage_tile<kTile>(Xs, V + (size_t)b * W * P, W, P, p0);
+  stage_commit();
+  for (int e = tid; e < W * Hp; e += kPwThreads) w1[e % W * Hp + e / W] = e / W < H ? Q1[e] : 0.f;
+  for (int e = tid; e < Hp * 16; e += kPwThreads) w2[e] = e / 16 < H && e % 16 < K ? Q2[(e % 16) * H + e / 16] : 0.f;
+  for (int e = tid; e < Hp; e += kPwThreads) b1[e] = e < H ? q1[e] : 0.f;
+  stage_wait();
+  __syncthreads();
+  Acc y;
+  y.zero();
+  float *mine = Hs + 16 * half * kTile;  // a thread reads and writes its own points of its half's channels only
+  for (int h0 = 16 * half; h0 < Hp; h0 += 32) {
+    Acc z;
+#pragma unroll
+    for (int o = 0; o < 8; ++o)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) z.v[u][o] = pack2(b1[h0 + 2 * o], b1[h0 + 2 * o + 1]);
+    mix16(z, Xs, w1 + h0, Hp, W, t);
+    acc_to_tile(z, mine, t);
+    const int mh = min(16, H - h0);
+#pragma unroll 1
+    for (int h = 0; h < mh; ++h) {
+      const size_t at = ((size_t)b * H + h0 + h) * P + p0 + t;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float *z1 = mine + h * kTile + t + 64 * u;
+        const float x = *z1, g = gelu(x);
+        *z1 = g;
+        if (p0 + t + 64 * u < P) {
+          Z[at + 64 * u] = x;
+          Hh[at + 64 * u] = g;
+        }
+      }
+    }
+    mix16(y, mine, w2 + h0 * 16, 16, max(mh, 0), t);
+  }
+  __syncthreads();
+  if (half) acc_to_tile(y, Hs, t);
+  __syncthreads();
+  if (!half) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+      if (k < K) {
+        const float bk = q2[k];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (p0 + t + 64 * u < P)
+            Y[((size_t)b * K + k) * P + p0 + t + 64 * u] = (y.get(u, k) + Hs[k * kTile + t + 64 * u]) + bk;
+      }
+  }
+}
+
+// Loss, first stage: block (slice, k, b) sums y u and y y over its slice of the points.
+constexpr int kLossSlice = 4096;
+__global__ void __launch_bounds__(256) loss_part_kernel(const float *__restrict__ Y, const float *__restrict__ T, int K,
+                                                        int P, float2 *part) {
+  __shared__ float r1[8], r2[8];
+  const int k = blockIdx.y, b = blockIdx.z;
+  const size_t base = ((size_t)b * K + k) * P;
+  const int p1 = min(P, (int)(blockIdx.x + 1) * kLossSlice);
+  float yu = 0.f, yy = 0.f;
+#pragma unroll 4
+  for (int p = blockIdx.x * kLossSlice + threadIdx.x; p < p1; p += 256) {
+    const float y = Y[base + p], u = T[base + p];
+    yu = fmaf(y, u, yu);
+    yy = fmaf(y, y, yy);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    yu += __shfl_xor_sync(0xffffffffu, yu, o);
+    yy += __shfl_xor_sync(0xffffffffu, yy, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    r1[threadIdx.x >> 5] = yu;
+    r2[threadIdx.x >> 5] = yy;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      yu += r1[w];
+      yy += r2[w];
+    }
+    part[((size_t)b * K + k) * gridDim.x + blockIdx.x] = make_float2(yu, yy);
+  }
+}
+// Second stage: loss_bk = 1 - (y.u)^2/(y.y) and the factors of dY = cu u + cy y.
+__global__ void loss_final_kernel(const float2 *__restrict__ part, int slices, int count, float scale, float *loss_bk,
+                                  float2 *coef) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= count) return;
+  float yu = 0.f, yy = 0.f;
+  for (int s = 0; s < slices; ++s) {
+    const float2 v = part[(size_t)e * slices + s];
+    yu += v.x;
+    yy += v.y;
+  }
+  yy = fmaxf(yy, 1e-30f);
+  loss_bk[e] = 1.f - yu * yu / yy;
+  coef[e] = make_float2(-2.f * yu / yy * scale, 2.f * yu * yu / (yy * yy) * scale);
+}
+
+// Projection, backward: dY = cu T + cy Y (written for the gradient of Q2), dH = Q2^T dY, dZ = dH gelu'(Z)
+// (written for the gradient of Q1), dV = Q1^T dZ for at most 32 channels per blockIdx.z, and the partial sums of
+// dq2, dq1 (z = 0) and of dV.  Hidden channels go 32 at a time.
+__global__ void __launch_bounds__(kPwThreads) proj_bwd_kernel(const float *__restrict__ Y, const float *__restrict__ T,
+                                                              const float2 *__restrict__ coef, const float *__restrict__ Z,
+                                                              int W, int H, int K, int P, const float *__restrict__ Q1,
+                                                              const float *__restrict__ Q2, float *dY, float *dZ,
+                                                              float *dV, float *part_k, float *part_h, float *part_w) {
+  extern __shared__ __align__(16) float sm[];
+  const int Hp = (H + 31) & ~31, c0 = blockIdx.z * 32, nc = min(32, W - c0);
+  float *Zs = sm;                  // [32][kTile]: Z of the group, then dZ; at the end dV
+  float *Ds = Zs + 32 * kTile;     // [32][kTile]: dH of the group
+  float *Ys = Ds + 32 * kTile;     // [K][kTile]: dY
+  float *w2 = Ys + K * kTile;      // [K][Hp]
+  float *w1 = w2 + K * Hp;         // [Hp][32]
+  const int tid = threadIdx.x, t = tid & 63, half = tid >> 6, b = blockIdx.y, p0 = blockIdx.x * kTile;
+  const bool first = blockIdx.z == 0;
+  const size_t blocks = (size_t)gridDim.x * gridDim.y, blk = (size_t)b * gridDim.x + blockIdx.x;
+  stage_tile<kTile>(Zs, Z + (size_t)b * H * P, min(32, H), P, p0);
+  stage_commit();
+  for (int e = tid; e < K * Hp; e += kPwThreads) w2[e] = e % Hp < H ? Q2[(e / Hp) * H + e % Hp] : 0.f;
+  for (int e = tid; e < Hp * 32; e += kPwThreads)
+    w1[e] = (e >> 5) < H && (e & 31) < nc ? Q1[(e >> 5) * W + c0 + (e & 31)] : 0.f;
+#pragma unroll 2
+  for (int k = half; k < K; k += 2) {
+    const float2 cf = __ldg(coef + b * K + k);
+    const size_t at = ((size_t)b * K + k) * P + p0 + t;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float d = 0.f;
+      if (p0 + t + 64 * u < P) {
+        d = cf.x * __ldg(T + at + 64 * u) + cf.y * __ldg(Y + at + 64 * u);
+        if (first) dY[at + 64 * u] = d;
+      }
+      Ys[k * kTile + t + 64 * u] = d;
+    }
+  }
+  if (first) tile_sums(Ys, K, part_k + blk, blocks);
+  Acc g;
+  g.zero();
+  float *zh = Zs + 16 * half * kTile + t, *dh = Ds + 16 * half * kTile + t;
+  for (int g0 = 0; g0 < H; g0 += 32) {
+    stage_wait();
+    __syncthreads();
+    const int h0 = g0 + 16 * half, mh = min(16, H - h0);
+    {
+      Acc d;
+      d.zero();
+      mix16(d, Ys, w2 + h0, Hp, K, t);
+      acc_to_tile(d, Ds + 16 * half * kTile, t);
+    }
+    // a thread's own points and channels: no barrier
+#pragma unroll 1
+    for (int h = 0; h < mh; ++h) {
+      const size_t at = ((size_t)b * H + h0 + h) * P + p0 + t;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float x = dh[h * kTile + 64 * u] * gelu_grad(zh[h * kTile + 64 * u]);  // dY = 0 past P
+        zh[h * kTile + 64 * u] = x;
+        if (first && p0 + t + 64 * u < P) dZ[at + 64 * u] = x;
+      }
+    }
+    const int mg = min(32, H - g0);
+    if (first) tile_sums(Zs, mg, part_h + (size_t)g0 * blocks + blk, blocks);
+    else __syncthreads();
+    mix16(g, Zs, w1 + g0 * 32 + 16 * half, 32, mg, t);
+    __syncthreads();
+    if (g0 + 32 < H) {
+      stage_tile<kTile>(Zs, Z + ((size_t)b * H + g0 + 32) * P, min(32, H - g0 - 32), P, p0);
+      stage_commit();
+    }
+  }
+  acc_to_tile(g, Zs + 16 * half * kTile, t);
+#pragma unroll 2
+  for (int o = 0; o < min(16, nc - 16 * half); ++o) {
+    const size_t at = ((size_t)b * W + c0 + 16 * half + o) * P + p0 + t;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p0 + t + 64 * u < P) dV[at + 64 * u] = zh[o * kTile + 64 * u];  // zero past P
+  }
+  tile_sums(Zs, nc, part_w + (size_t)c0 * blocks + blk, blocks);
+}
+
+// C[z] (M x M) = S^T X[z] S for the fields z = blockIdx.x of N x N points, 128 columns per block (blockIdx.y): the
+// rows stream through a ring of shared-memory stages (32 rows of X and of S each), each warp forms T1 = S^T X
+// over its rows with four columns per lane (they share the loads of S), the warps' shares are added in order,
+// and the block multiplies by S.  The blocks of a field leave their shares in work, and the last to finish adds
+// them in order (count: one zeroed word per field, zero again afterwards).  Bound: HBM, one read of X.
+// 128 fields of 512 x 512: 56 us (134 MB, 21 us); with loads into registers instead of the stages 130 to 186 us.
+constexpr int kModeThreads = 256;
+constexpr int kModeCols = 128;
+constexpr int kModeWarps = kModeThreads / 32;
+constexpr int kModeRows = 32;    // rows of a stage
+constexpr int kModeStages = 3;
+constexpr int kModeStage = kModeRows * (kModeCols + kModes);  // floats of a stage
+constexpr size_t kModeSmem = sizeof(float) * kModeStages * kModeStage;
+__global__ void __launch_bounds__(kModeThreads, 2) modes_kernel(const float *__restrict__ X, const float *__restrict__ Sp,
+                                                                int N, int M, float *C, float *work, unsigned *count) {
+  extern __shared__ __align__(16) float sm[];  // the stages; then the warps' shares of T1, half of them at a time
+  static_assert(kModeWarps / 2 * kModes * kModeCols <= kModeStages * kModeStage, "T1 shares fit the stages");
+  __shared__ int last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int j0 = blockIdx.y * kModeCols, nst = (N + kModeRows - 1) / kModeRows;
+  const float *F = X + (size_t)blockIdx.x * N * N;
+  const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(sm);
+  const bool wide = (N & 3) == 0 && ((uintptr_t)X & 15) == 0;
+  auto load = [&](int st) {
+    if (st < nst) {
+      const int i0 = st * kModeRows;
+      const uint32_t xs = sm0 + 4u * (uint32_t)(st % kModeStages * kModeStage), ss = xs + 4u * kModeRows * kModeCols;
+      if (wide) {
+        for (int e = tid; e < kModeRows * kModeCols / 4; e += kModeThreads) {
+          const int i = i0 + (e >> 5), j = j0 + 4 * (e & 31);
+          const bool in = i < N && j < N;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(xs + 16u * (uint32_t)e),
+                       "l"(F + (in ? (size_t)i * N + j : 0)), "r"(in ? 16 : 0)
+                       : "memory");
+        }
+      } else {
+        for (int e = tid; e < kModeRows * kModeCols; e += kModeThreads) {
+          const int i = i0 + (e >> 7), j = j0 + (e & 127);
+          const bool in = i < N && j < N;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(xs + 4u * (uint32_t)e),
+                       "l"(F + (in ? (size_t)i * N + j : 0)), "r"(in ? 4 : 0)
+                       : "memory");
+        }
+      }
+      if (tid < kModeRows * kModes / 4) {
+        const int i = i0 + (tid >> 2);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ss + 16u * (uint32_t)tid),
+                     "l"(Sp + (i < N ? (size_t)i * kModes + 4 * (tid & 3) : 0)), "r"(i < N ? 16 : 0)
+                     : "memory");
+      }
+    }
+    stage_commit();
+  };
+  unsigned long long acc[4][kModes / 2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int q = 0; q < kModes / 2; ++q) acc[u][q] = 0ull;
+#pragma unroll
+  for (int st = 0; st < kModeStages - 1; ++st) load(st);
+  for (int st = 0; st < nst; ++st) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kModeStages - 2) : "memory");
+    __syncthreads();  // stage st has landed, stage st - 1 is consumed
+    load(st + kModeStages - 1);
+    const float *xs = sm + st % kModeStages * kModeStage, *ss = xs + kModeRows * kModeCols;
+#pragma unroll
+    for (int r = 0; r < kModeRows / kModeWarps; ++r) {
+      const int row = r * kModeWarps + warp;
+      const float4 x = *reinterpret_cast<const float4 *>(xs + row * kModeCols + 4 * lane);
+      const unsigned long long xx[4] = {pack2(x.x, x.x), pack2(x.y, x.y), pack2(x.z, x.z), pack2(x.w, x.w)};
+#pragma unroll
+      for (int q = 0; q < kModes / 4; ++q) {
+        const ulonglong2 s2 = reinterpret_cast<const ulonglong2 *>(ss + row * kModes)[q];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          fma2(acc[u][2 * q], s2.x, xx[u]);
+          fma2(acc[u][2 * q + 1], s2.y, xx[u]);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  // T1 of the 128 columns: warps 4..7 leave theirs, warps 0..3 add theirs, then the four sums in order
+  auto row4 = [&](int w, int q) { return reinterpret_cast<float4 *>(sm + (w * kModes + q) * kModeCols + 4 * lane); };
+  auto value = [&](int q, int u) {
+    const float2 f = unpack2(acc[u][q >> 1]);
+    return q & 1 ? f.y : f.x;
+  };
+  if (warp >= kModeWarps / 2)
+#pragma unroll
+    for (int q = 0; q < kModes; ++q)
+      *row4(warp - kModeWarps / 2, q) = make_float4(value(q, 0), value(q, 1), value(q, 2), value(q, 3));
+  __syncthreads();
+  if (warp < kModeWarps / 2)
+#pragma unroll
+    for (int q = 0; q < kModes; ++q) {
+      float4 v = *row4(warp, q);
+      v.x += value(q, 0);
+      v.y += value(q, 1);
+      v.z += value(q, 2);
+      v.w += value(q, 3);
+      *row4(warp, q) = v;
+    }
+  __syncthreads();
+  for (int e = tid; e < kModes * kModeCols; e += kModeThreads) {
+    float s = sm[e];
+#pragma unroll
+    for (int h = 1; h < kModeWarps / 2; ++h) s += sm[h * kModes * kModeCols + e];
+    sm[e] = s;
+  }
+  __syncthreads();
+  const int k = tid >> 4, m = tid & 15, jn = min(kModeCols, N - j0);
+  float part[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int j = 0; j < jn; j += 4) {
+    const float4 v = *reinterpret_cast<const float4 *>(sm + k * kModeCols + j);  // zeros past N
+    const float *s = Sp + (size_t)(j0 + j) * kModes + m;
+    part[0] = fmaf(v.x, __ldg(s), part[0]);
+    if (j + 1 < jn) part[1] = fmaf(v.y, __ldg(s + kModes), part[1]);
+    if (j + 2 < jn) part[2] = fmaf(v.z, __ldg(s + 2 * kModes), part[2]);
+    if (j + 3 < jn) part[3] = fmaf(v.w, __ldg(s + 3 * kModes), part[3]);
+  }
+  const float total = (part[0] + part[1]) + (part[2] + part[3]);
+  float *out = C + (size_t)blockIdx.x * M * M + k * M + m;
+  const bool mine = k < M && m < M;
+  if (gridDim.y == 1) {
+    if (mine) *out = total;
+    return;
+  }
+  float *w = work + (size_t)blockIdx.x * gridDim.y * kModeThreads;
+  w[(size_t)blockIdx.y * kModeThreads + tid] = total;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(count + blockIdx.x, 1u) == gridDim.y - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  float s = 0.f;
+#pragma unroll 4
+  for (unsigned q = 0; q < gridDim.y; ++q) s += __ldcg(w + (size_t)q * kModeThreads + tid);
+  if (mine) *out = s;
+  if (tid == 0) count[blockIdx.x] = 0;
+}
+
+// Per-mode channel mix and the first half of the way back to the grid, one block per (channel x, sample b), one
+// thread per mode q = (k, m): D(q) = sum_y R(...) in(b, y, q) with R(o, c, q) at (o W + c) M2 + q (transposed = 0:
+// x = o, y = c, forward; 1: x = c, y = o, backward), then T2(b, x, i, m) = sum_k S(i, k) D(k, m) for every image
+// row i.  Blocks past W B form dR(o, c, q) = sum_b dD(b, o, q) C(b, c, q) instead (backward only).
+__global__ void __launch_bounds__(256) mode_mix_kernel(const float *__restrict__ R, const float *__restrict__ in,
+                                                       const float *__restrict__ Sp, float *T2, int B, int W, int N, int M,
+                                                       int transposed, const float *__restrict__ C, float *dR) {
+  __shared__ float D[kModes * kModes];
+  const int M2 = M * M, q = threadIdx.x;
+  int x = blockIdx.x;
+  if (x < W * B) {
+    const int b = x / W;
+    x %= W;
+    float acc = 0.f;
+    if (q < M2) {
+#pragma unroll 8
+      for (int y = 0; y < W; ++y)
+        acc = fmaf(__ldg(R + ((size_t)(transposed ? y * W + x : x * W + y)) * M2 + q),
+                   __ldg(in + ((size_t)b * W + y) * M2 + q), acc);
+      D[q] = acc;
+    }
+    __syncthreads();
+    float *out = T2 + ((size_t)b * W + x) * N * M;
+    const int m = q & 15;
+    if (m < M) {
+      float d[kModes];
+#pragma unroll
+      for (int k = 0; k < kModes; ++k) d[k] = k < M ? D[k * M + m] : 0.f;
+      for (int i = q >> 4; i < N; i += 16) {
+        const float4 *s = reinterpret_cast<const float4 *>(Sp + (size_t)i * kModes);
+        float t = 0.f;
+#pragma unroll
+        for (int k = 0; k < kModes; k += 4) {
+          const float4 v = __ldg(s + k / 4);
+          t = fmaf(v.x, d[k], t);
+          t = fmaf(v.y, d[k + 1], t);
+          t = fmaf(v.z, d[k + 2], t);
+          t = fmaf(v.w, d[k + 3], t);
+        }
+        out[i * M + m] = t;
+      }
+    }
+    return;
+  }
+  if (q >= M2) return;
+  x -= W * B;  // o W + c
+  const int o = x / W, c = x % W;
+  float s = 0.f;
+#pragma unroll 4
+  for (int b = 0; b < B; ++b)
+    s = fmaf(__ldg(in + ((size_t)b * W + o) * M2 + q), __ldg(C + ((size_t)b * W + c) * M2 + q), s);
+  dR[(size_t)x * M2 + q] = s;
+}
+
+// Bias gradients from the blocks' partial sums: block s sums row s of part and stores it at grads[off].
+struct BiasRows {
+  int count;                 // tensors
+  int first[20];             // first row of each
+  int blocks[20];            // partial sums per row
+  long long at[20];          // element of the first partial sum of each
+  long long off[20];         // offset in the gradient array
+};
+__global__ void __launch_bounds__(128) bias_rows_kernel(const float *__restrict__ part, BiasRows r, float *grads) {
+  __shared__ float red[128];
+  int t = 0;
+  while (t + 1 < r.count && (int)blockIdx.x >= r.first[t + 1]) ++t;
+  const int c = blockIdx.x - r.first[t], n = r.blocks[t];
+  const float *p = part + r.at[t] + (size_t)c * n;
+  float s = 0.f;
+  for (int e = threadIdx.x; e < n; e += 128) s += p[e];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = 64; w > 0; w >>= 1) {
+    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) grads[r.off[t] + c] = red[0];
+}
+
+}  // namespace neural
+}  // namespace b200
