@@ -381,79 +381,112 @@ __global__ void dot_partial_kernel(const double *__restrict__ X, int ldx, int nx
   }
 }
 
-// Gram block M = Y^T X for up to T x T column pairs per CTA row, T = 16 TM (blockIdx.y, blockIdx.z
-// select the T-column blocks of Y and X; TM is chosen from the block width so that narrow blocks do
-// not pay for padding).  The CTA's rows are staged in 32-row panels in shared memory, the next panel
-// is loaded into registers while the current one is consumed, and thread (ty, tx) of a 16 x 16 layout
-// accumulates the TM x TM pairs (TM ty + a, TM tx + b) in row order.
-// partial[blk * (nx*ny) + (i + j*ny)] as dot_partial_kernel writes it.
-constexpr int kGramRows = 32;
-template <int TM>
-__global__ void __launch_bounds__(256) gram_partial_kernel(const double *__restrict__ X, int ldx, int nx,
-                                                           const double *__restrict__ Y, int ldy, int ny, int n,
-                                                           double *partial) {
-  constexpr int T = 16 * TM;
-  constexpr int kLoads = kGramRows * T / 256;  // elements of each operand a thread stages per panel
-  __shared__ double Xs[kGramRows][T + 1], Ys[kGramRows][T + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int y0 = blockIdx.y * T, x0 = blockIdx.z * T;
-  const int cy = min(T, ny - y0), cx = min(T, nx - x0);
-  const long long rows_per = (n + gridDim.x - 1) / gridDim.x;
-  const long long r0 = (long long)blockIdx.x * rows_per;
-  const long long r1 = min((long long)n, r0 + rows_per);
-  double acc[TM][TM];
-#pragma unroll
-  for (int a = 0; a < TM; ++a)
-#pragma unroll
-    for (int b = 0; b < TM; ++b) acc[a][b] = 0.0;
-  double xr[kLoads], yr[kLoads];
-  // column-major loads: 32 consecutive rows of one column per warp
-  auto load = [&](long long p0, int pr) {
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int e = threadIdx.x + 256 * u;
-      const int r = e % kGramRows, c = e / kGramRows;
-      xr[u] = (r < pr && c < cx) ? X[(size_t)(x0 + c) * ldx + p0 + r] : 0.0;
-      yr[u] = (r < pr && c < cy) ? Y[(size_t)(y0 + c) * ldy + p0 + r] : 0.0;
+__device__ __forceinline__ void dmma_m16n8k16(double (&d)[4], const double (&a)[8], const double (&b)[4]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, "
+      "{%12,%13,%14,%15}, {%0,%1,%2,%3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
+        "d"(b[1]), "d"(b[2]), "d"(b[3]));
+}
+
+// Gram block M = Y^T X on the FP64 MMA path (mma.sync.m16n8k16.f64; tcgen05 has no FP64 kind), up to 64 columns of
+// each side per CTA (blockIdx.y, blockIdx.z select the 64-column blocks of Y and X).  The CTA's rows stream
+// through a ring of kGramStages stages of 32 rows with asynchronous copies (column stride 36 doubles, 4 mod 16: the
+// fragment loads of a half warp hit distinct banks).  The 8 warps are 16-column strips of Y (STRIPS) times the two
+// 16-row halves of a stage times, where warps are left, halves of X's 8-column tiles; the row halves meet in
+// shared memory at the end.  SELF: X is Y, staged once.  Fragments (g = lane / 4, t = lane % 4): A = Y^T, element e
+// at row g + 8 (e % 2), depth t + 4 (e / 2); B element e at depth t + 4 e, column g; D element e at row
+// g + 8 (e / 2), column 2 t + e % 2.  partial[cta * nx ny + i + j ny].
+//
+// Bound: for 48 x 48 columns of n = 262,144 rows 201 MB (31 us) and 1.2 GFLOP (33 us at the 37 TFLOP/s of this
+// shape).  A whole b200_bv_dot of that size takes 110 us with its read-back, 148 us with a CUDA-core kernel of register
+// tiles, which was bound by its shared-memory reads.
+constexpr int kGramRows = 32;    // rows per stage
+constexpr int kGramLd = 36;      // doubles per staged column
+constexpr int kGramStages = 3;
+template <int STRIPS, bool SELF>
+__global__ void __launch_bounds__(256) gram_mma_kernel(const double *__restrict__ X, int ldx, int nx,
+                                                       const double *__restrict__ Y, int ldy, int ny, int n,
+                                                       double *partial) {
+  extern __shared__ __align__(16) double gsm[];
+  constexpr int NH = STRIPS <= 2 ? 2 : 1;   // halves of X's column tiles
+  constexpr int TILES = 8 / NH;             // 8-column tiles of X a warp holds
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int y0 = blockIdx.y * 64, x0 = blockIdx.z * 64;
+  const int cy = min(16 * STRIPS, ny - y0), cx = min(64, nx - x0);
+  const int cyp = 16 * STRIPS, cxp = SELF ? 0 : (cx + 7) & ~7;  // staged columns (zero past cy, cx)
+  const int stage = (cyp + cxp) * kGramLd;
+  const int strip = warp % STRIPS, kg = warp / STRIPS % 2, nh = warp / (2 * STRIPS);
+  const bool active = nh < NH;
+  const int tiles = (cx + 7) / 8, j0 = nh * ((tiles + NH - 1) / NH), j1 = min(tiles, j0 + (tiles + NH - 1) / NH);
+  const long long rows_per = ((long long)(n + gridDim.x - 1) / gridDim.x + kGramRows - 1) / kGramRows * kGramRows;
+  const long long r0 = (long long)blockIdx.x * rows_per, r1 = min((long long)n, r0 + rows_per);
+  const int nst = r1 > r0 ? (int)((r1 - r0 + kGramRows - 1) / kGramRows) : 0;
+  const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(gsm);
+  auto load = [&](int st) {
+    if (st < nst) {
+      const long long p0 = r0 + (long long)st * kGramRows;
+      const uint32_t base = sm0 + 8u * (uint32_t)(st % kGramStages * stage);
+      const int rows = (int)min((long long)kGramRows, r1 - p0);
+      for (int e = tid; e < (cyp + cxp) * (kGramRows / 2); e += 256) {
+        const int c = e / (kGramRows / 2), r = 2 * (e % (kGramRows / 2));
+        const bool isy = c < cyp;
+        const int col = isy ? c : c - cyp;
+        const bool in = col < (isy ? cy : cx) && r < rows;
+        const double *src = isy ? Y + (size_t)(y0 + (in ? col : 0)) * ldy : X + (size_t)(x0 + (in ? col : 0)) * ldx;
+        const uint32_t dst = base + 8u * (uint32_t)(c * kGramLd + r);
+        const int bytes = in ? min(16, 8 * (rows - r)) : 0;  // columns are 16-byte aligned (even leading dimension)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src + p0 + (in ? r : 0)), "r"(bytes)
+                     : "memory");
+      }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  long long p0 = r0;
-  int pr = p0 < r1 ? (int)min((long long)kGramRows, r1 - p0) : 0;
-  if (pr > 0) load(p0, pr);
-  while (pr > 0) {
+  double acc[TILES][4];
 #pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int e = threadIdx.x + 256 * u;
-      const int r = e % kGramRows, c = e / kGramRows;
-      Xs[r][c] = xr[u];
-      Ys[r][c] = yr[u];
+  for (int j = 0; j < TILES; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
+#pragma unroll
+  for (int st = 0; st < kGramStages - 1; ++st) load(st);
+  for (int st = 0; st < nst; ++st) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kGramStages - 2) : "memory");
+    __syncthreads();  // stage st has landed, stage st - 1 is consumed
+    load(st + kGramStages - 1);
+    if (active) {
+      const double *ys = gsm + st % kGramStages * stage, *xs = SELF ? ys : ys + cyp * kGramLd;
+      const int k0 = 16 * kg;
+      double a[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] = ys[(16 * strip + g + 8 * (e & 1)) * kGramLd + k0 + t + 4 * (e >> 1)];
+#pragma unroll
+      for (int j = 0; j < TILES; ++j) {
+        if (j0 + j < j1) {
+          double b[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) b[e] = xs[(8 * (j0 + j) + g) * kGramLd + k0 + t + 4 * e];
+          dmma_m16n8k16(acc[j], a, b);
+        }
+      }
     }
-    __syncthreads();
-    const long long pn = p0 + kGramRows;
-    const int prn = pn < r1 ? (int)min((long long)kGramRows, r1 - pn) : 0;
-    if (prn > 0) load(pn, prn);  // in flight while this panel is consumed
-    for (int r = 0; r < pr; ++r) {
-      double yv[TM], xv[TM];
-#pragma unroll
-      for (int a = 0; a < TM; ++a) yv[a] = Ys[r][TM * ty + a];
-#pragma unroll
-      for (int b = 0; b < TM; ++b) xv[b] = Xs[r][TM * tx + b];
-#pragma unroll
-      for (int a = 0; a < TM; ++a)
-#pragma unroll
-        for (int b = 0; b < TM; ++b) acc[a][b] = fma(yv[a], xv[b], acc[a][b]);
-    }
-    __syncthreads();
-    p0 = pn;
-    pr = prn;
   }
-  const int npairs = nx * ny;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  // the second row half's sums through shared memory, [strip, half][element][lane]
+  double *other = gsm + (size_t)(strip * NH + (active ? nh : 0)) * TILES * 4 * 32 + lane;
+  if (active && kg == 1)
 #pragma unroll
-  for (int a = 0; a < TM; ++a)
+    for (int j = 0; j < TILES; ++j)
 #pragma unroll
-    for (int b = 0; b < TM; ++b) {
-      const int i = TM * ty + a, j = TM * tx + b;
-      if (i < cy && j < cx) partial[(size_t)blockIdx.x * npairs + (y0 + i) + (size_t)(x0 + j) * ny] = acc[a][b];
+      for (int e = 0; e < 4; ++e) other[(j * 4 + e) * 32] = acc[j][e];
+  __syncthreads();
+  if (!active || kg != 0) return;
+  double *out = partial + (size_t)blockIdx.x * nx * ny;
+#pragma unroll
+  for (int j = 0; j < TILES; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = 16 * strip + g + 8 * (e >> 1), col = 8 * (j0 + j) + 2 * t + (e & 1);
+      if (j0 + j < j1 && i < cy && col < cx) out[(y0 + i) + (size_t)(x0 + col) * ny] = acc[j][e] + other[(j * 4 + e) * 32];
     }
 }
 
@@ -466,15 +499,6 @@ __global__ void __launch_bounds__(256) gram_partial_kernel(const double *__restr
 // element e at row g + 8 (e / 2), column 2 t + e % 2.  Partial sums partial[cta][M1 then M2], each (i + j nc).
 constexpr int kDualRows = 32;  // rows per staged chunk
 constexpr int kDualLd = 36;    // doubles per staged column
-__device__ __forceinline__ void dmma_m16n8k16(double (&d)[4], const double (&a)[8], const double (&b)[4]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, "
-      "{%12,%13,%14,%15}, {%0,%1,%2,%3};"
-      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
-        "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
-
 template <int NMB>
 __global__ void __launch_bounds__(256) gram_dual_mma_kernel(const double *__restrict__ X, int ldx,
                                                             const double *__restrict__ Y, int ldy, int nc, int n,
@@ -1059,25 +1083,43 @@ cudaError_t multvec_launch(const double *X, int ldx, int n, int k, const double 
   return cudaGetLastError();
 }
 
+template <int STRIPS, bool SELF>
+cudaError_t gram_mma_launch(const double *X, int ldx, int nx, const double *Y, int ldy, int ny, int n, double *work,
+                            int blocks, cudaStream_t stream) {
+  const cudaError_t e = allow_max_dynamic_smem(gram_mma_kernel<STRIPS, SELF>);
+  if (e != cudaSuccess) return e;
+  const int cx = nx < 64 ? (nx + 7) & ~7 : 64;
+  size_t smem = sizeof(double) * kGramStages * kGramLd * (size_t)(16 * STRIPS + (SELF ? 0 : cx));
+  const size_t exchange = sizeof(double) * 32 * 32 * (size_t)STRIPS;
+  if (smem < exchange) smem = exchange;
+  const dim3 grid(blocks, (ny + 63) / 64, (nx + 63) / 64);
+  gram_mma_kernel<STRIPS, SELF><<<grid, 256, smem, stream>>>(X, ldx, nx, Y, ldy, ny, n, work);
+  return cudaGetLastError();
+}
+
 cudaError_t dot_launch(const double *X, int ldx, int nx, const double *Y, int ldy, int ny, int n, double *M, int ldm,
                        double *work, int work_len, cudaStream_t stream, int ctas_per_sm) {
   if (nx <= 0 || ny <= 0) return cudaSuccess;
   const int npairs = nx * ny;
   int blocks = num_sms() * (ctas_per_sm > 0 ? ctas_per_sm : 1);
+  const int most = (n + 4 * kGramRows - 1) / (4 * kGramRows);  // at least four stages of rows a block
+  if (npairs >= 64 && blocks > most) blocks = most;
   if (blocks * npairs > work_len) blocks = work_len / npairs;
   if (blocks < 1) return cudaErrorInvalidValue;
   if (npairs >= 64) {
-    // register-tiled Gram blocks: both blocks of columns read once per CTA row range
-    const int w = nx > ny ? nx : ny;
-    const int tm = w > 48 ? 4 : (w + 15) / 16;
-    const int T = 16 * tm;
-    const dim3 grid(blocks, (ny + T - 1) / T, (nx + T - 1) / T);
-    switch (tm) {
-      case 1: gram_partial_kernel<1><<<grid, 256, 0, stream>>>(X, ldx, nx, Y, ldy, ny, n, work); break;
-      case 2: gram_partial_kernel<2><<<grid, 256, 0, stream>>>(X, ldx, nx, Y, ldy, ny, n, work); break;
-      case 3: gram_partial_kernel<3><<<grid, 256, 0, stream>>>(X, ldx, nx, Y, ldy, ny, n, work); break;
-      default: gram_partial_kernel<4><<<grid, 256, 0, stream>>>(X, ldx, nx, Y, ldy, ny, n, work); break;
+    const bool self = X == Y && ldx == ldy && nx == ny && nx <= 64;
+    const int strips = ny > 48 ? 4 : (ny + 15) / 16;
+    cudaError_t e;
+    switch (strips) {
+#define B200_GRAM_CASE(S)                                                                                         case S:                                                                                                           e = self ? gram_mma_launch<S, true>(X, ldx, nx, Y, ldy, ny, n, work, blocks, stream)                                     : gram_mma_launch<S, false>(X, ldx, nx, Y, ldy, ny, n, work, blocks, stream);                          break;
+      B200_GRAM_CASE(1)
+      B200_GRAM_CASE(2)
+      B200_GRAM_CASE(3)
+      default:
+      B200_GRAM_CASE(4)
+#undef B200_GRAM_CASE
     }
+    if (e != cudaSuccess) return e;
   } else {
     dot_partial_kernel<<<blocks, 256, 0, stream>>>(X, ldx, nx, Y, ldy, ny, n, work);
   }

@@ -1460,7 +1460,7 @@ b200_status bv_dot_pair(b200_bv W, b200_bv Z, double *MA, double *MB, int ldm) {
   B200_ARG_CHECK(W->k - W->l == nc && ldm >= Z->k && ldm >= W->k, "BVDot pair: column ranges differ");
   if (nc <= 0) return B200_OK;
   const size_t sq = (size_t)nc * nc;
-  const int cps = dot_ctas_per_sm(nc, nc);
+  const int cps = nc <= 64 ? kDualCtasPerSm : dot_ctas_per_sm(nc, nc);
   B200_CHECK(bv_reserve(Z, 2 * sq, 2 * sq * num_sms_host() * cps));
   cudaError_t e = dot_dual_launch(col(W, W->l), W->ld, col(Z, Z->l), Z->ld, nc, Z->n, Z->qbuf, Z->red, Z->red_len,
                                   Z->stream, cps);
