@@ -96,18 +96,43 @@ __device__ void cta_spmv(const BProblem &P, const int *__restrict__ rowptr, cons
   const int *rp = rowptr + P.rp_off;
   const int *ci = colind + P.nnz_off;
   const double *va = vals + P.nnz_off;
+  // every value and column index of a tile in flight together, then every x; the next tile's entries load
+  // while the current tile gathers and sums (62,000 -> 27,000 cycles at n = 2,218)
+  constexpr int U = kWarpTileNnz / 32;
+  double a[U];
+  int c[U], mystart = 0;
+  int4 tile = make_int4(0, 0, 0, 0);
+  auto fetch = [&](int t) {
+    if (t >= P.ntiles) return;
+    tile = __ldg(tiles + P.tile_off + t);
+    mystart = lane < tile.y - tile.x ? __ldg(rp + tile.x + lane) : 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int q = tile.z + lane + 32 * u;
+      a[u] = q < tile.w ? __ldg(va + q) : 0.0;
+      c[u] = q < tile.w ? __ldg(ci + q) : -1;
+    }
+  };
+  fetch(wib);
   for (int t = wib; t < P.ntiles; t += T / 32) {
-    const int4 tile = tiles[P.tile_off + t];
-    const int r0 = tile.x, r1 = tile.y, nrows = r1 - r0, p0 = tile.z, p1 = tile.w;
-    const int mystart = (lane < nrows) ? rp[r0 + lane] : 0;
-    const int nxt = __shfl_down_sync(0xffffffffu, mystart, 1);
+    const int r0 = tile.x, nrows = tile.y - tile.x, p0 = tile.z, p1 = tile.w, start = mystart;
+    XT xv[U];
+    double av[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      xv[u] = c[u] >= 0 ? __ldcg(x + c[u]) : XT(0);
+      av[u] = a[u];
+    }
+    fetch(t + T / 32);
+    const int nxt = __shfl_down_sync(0xffffffffu, start, 1);
     const int myend = (lane + 1 < nrows) ? nxt : p1;
-    const int cnt = p1 - p0;
-    for (int q = lane; q < cnt; q += 32) prod[q] = __dmul_rn(va[p0 + q], (double)__ldcg(x + ci[p0 + q]));
+#pragma unroll
+    for (int u = 0; u < U; ++u) prod[lane + 32 * u] = __dmul_rn(av[u], (double)xv[u]);
     __syncwarp();
     if (lane < nrows) {
       double s = 0.0;
-      for (int q = mystart - p0; q < myend - p0; ++q) s = __dadd_rn(s, prod[q]);
+#pragma unroll 4
+      for (int q = start - p0; q < myend - p0; ++q) s = __dadd_rn(s, prod[q]);
       y[r0 + lane] = s;
     }
     __syncwarp();
@@ -115,48 +140,82 @@ __device__ void cta_spmv(const BProblem &P, const int *__restrict__ rowptr, cons
   __syncthreads();
 }
 
-// sh.c[i] = V(:,c0+i)' w for i < ncols (deterministic); w may be one of the columns.  Columns
-// go in groups of 8: per-thread partial sums in row order, a fixed shuffle tree per warp, the
-// warps added in order.
-template <int T>
-__device__ void cta_dots(const double *V, int ld, int n, int c0, int ncols, const double *w, BShared<T> &sh) {
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  if (threadIdx.x == 0) sh.bytes += 8ull * n * (ncols + 1);
-  for (int g0 = 0; g0 < ncols; g0 += 8) {
-    const int gn = min(8, ncols - g0);
-    double acc[8];
+// Lane l < CB returns the sum over the lanes of acc[l] (a halving exchange).
+template <int CB>
+__device__ __forceinline__ double bcolumn_sums(const double (&acc)[CB], int lane) {
+  double v[32];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.0;
-    for (int r = threadIdx.x; r < n; r += T) {
-      const double wr = __ldcg(w + r);
+  for (int i = 0; i < 32; ++i) v[i] = i < CB ? acc[i < CB ? i : 0] : 0.0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (i < gn) acc[i] = fma(__ldcg(V + r + (size_t)(c0 + g0 + i) * ld), wr, acc[i]);
-    }
+  for (int half = 16; half > 0; half >>= 1) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const double v = bwarp_sum(acc[i]);
-      if (lane == 0) sh.red[wib][g0 + i] = v;
+    for (int i = 0; i < half; ++i) {
+      const bool up = (lane & half) != 0;
+      const double keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
     }
   }
-  __syncthreads();
-  if (threadIdx.x < ncols) {
-    double sacc = 0.0;
-    for (int w2 = 0; w2 < T / 32; ++w2) sacc += sh.red[w2][threadIdx.x];
-    sh.c[threadIdx.x] = sacc;
-  }
-  __syncthreads();
+  return v[0];
 }
 
-// w -= V(:,0:ncols) coef
-template <int T>
-__device__ void cta_update(const double *V, int ld, int n, int ncols, const double *coef, double *w) {
+// One sweep over the rows: any of UPDATE w <- (w - V(:,0:ncols) coef) scale and DOT sh.c[i] = V(:,i)' w',
+// sh.c[ncols] = w' w' (deterministic: per-thread sums in row order, a fixed exchange per warp, the warps in
+// order).  A thread holds its row of all columns (CB >= ncols) in registers, so the update and the dot share
+// one read of V and every load of a row is in flight at once.  Measured per column of n = 2,218 (256 threads,
+// about 18 columns): 45,000 cycles, where eight columns at a time with update and dot each reading V took
+// 103,000.  Batches: 192 problems n ~ U[500, 4000] 71.6 -> 38.1 ms, 4096 problems n ~ U[500, 20000] 6.9 -> 5.5 s.
+// Called, not inlined: the sixteen copies that a column would hold overflow the instruction cache.
+template <int T, int CB>
+__device__ __noinline__ void cta_sweep_cb(const double *V, int ld, int n, int ncols, double *w, const double *coef,
+                                             bool update, bool dot, double scale, BShared<T> &sh) {
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  double acc[CB], self = 0.0;
+#pragma unroll
+  for (int i = 0; i < CB; ++i) acc[i] = 0.0;
   for (int r = threadIdx.x; r < n; r += T) {
-    double acc = 0.0;
-    for (int i = 0; i < ncols; ++i) acc = fma(__ldcg(V + r + (size_t)i * ld), coef[i], acc);
-    w[r] = __ldcg(w + r) - acc;
+    double v[CB];
+    double wr = __ldcg(w + r);
+#pragma unroll
+    for (int i = 0; i < CB; ++i) v[i] = i < ncols ? __ldcg(V + r + (size_t)i * ld) : 0.0;
+    if (update) {
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int i = 0; i < CB; ++i)
+        if (i < ncols) s[i & 3] = fma(v[i], coef[i], s[i & 3]);
+      wr = (wr - ((s[0] + s[1]) + (s[2] + s[3]))) * scale;
+      w[r] = wr;
+    }
+    if (dot) {
+#pragma unroll
+      for (int i = 0; i < CB; ++i) acc[i] = fma(v[i], wr, acc[i]);
+      self = fma(wr, wr, self);
+    }
   }
-  __syncthreads();
+  if (dot) {
+    const double mine = bcolumn_sums<CB>(acc, lane);
+    self = bwarp_sum(self);
+    if (lane < ncols) sh.red[wib][lane] = mine;
+    if (lane == 0) sh.red[wib][ncols] = self;
+  }
+  __syncthreads();  // also: coef (sh.c) is consumed
+  if (dot) {
+    if (threadIdx.x <= ncols) {
+      double sacc = 0.0;
+      for (int w2 = 0; w2 < T / 32; ++w2) sacc += sh.red[w2][threadIdx.x];
+      sh.c[threadIdx.x] = sacc;
+    }
+    __syncthreads();
+  }
+}
+
+template <int T>
+__device__ void cta_sweep(const double *V, int ld, int n, int ncols, double *w, const double *coef, bool update, bool dot,
+                          double scale, BShared<T> &sh) {
+  if (threadIdx.x == 0) sh.bytes += 8ull * n * (ncols + 1 + (update ? 1 : 0));
+  if (ncols <= 8) cta_sweep_cb<T, 8>(V, ld, n, ncols, w, coef, update, dot, scale, sh);
+  else if (ncols <= 16) cta_sweep_cb<T, 16>(V, ld, n, ncols, w, coef, update, dot, scale, sh);
+  else if (ncols <= 24) cta_sweep_cb<T, 24>(V, ld, n, ncols, w, coef, update, dot, scale, sh);
+  else cta_sweep_cb<T, 32>(V, ld, n, ncols, w, coef, update, dot, scale, sh);
 }
 
 template <int T>
@@ -185,56 +244,59 @@ __device__ void cta_random(double *w, int n, uint64_t seed, uint64_t stream_id) 
 // h[0..j-1] holds the coefficients, *norm the norm of the new column, *lindep the flag.
 // The column is then scaled by 1/norm unless the norm is 0 or 1 (BVOrthonormalizeColumn).
 template <int T>
-__device__ void cta_orthonormalize(double *V, int ld, int n, int j, double eta, double *h, double *norm, int *lindep,
+__device__ __noinline__ void cta_orthonormalize(double *V, int ld, int n, int j, double eta, double *h, double *norm, int *lindep,
                                    int *err, BShared<T> &sh) {
   double *w = V + (size_t)j * ld;
   for (int i = 0; i < j; ++i) h[i] = 0.0;
-  int more = 1, passes = 0;
-  while (more) {
-    cta_dots<T>(V, ld, n, 0, j + 1, w, sh);  // includes w against itself
-    for (int i = 0; i < j; ++i) h[i] += sh.c[i];
-    cta_update<T>(V, ld, n, j, sh.c, w);
-    if (threadIdx.x == 0 && j > 0) sh.bytes += 8ull * n * (j + 2);
-    // thread 0: the Pythagorean estimate of the new norm (bvorthog.c:124-127)
-    if (threadIdx.x == 0) {
-      const double self = sh.c[j];
-      if (self < 0.0) sh.flag[2] = 1;
-      const double onrm = sqrt(self < 0.0 ? 0.0 : self);
-      double sum = 0.0;
-      for (int i = 0; i < j; ++i) sum += sh.c[i] * sh.c[i];
-      const double est = onrm * onrm - sum;
-      sh.scal[0] = onrm;
-      sh.scal[1] = est;
-      sh.flag[0] = est <= 0.0;
+  // The passes of gs_column_kernel: the update of a pass shares a sweep with the dot of the next (or of the
+  // explicit norm), and the last update carries the scaling.  Every thread takes the same decisions.
+  cta_sweep<T>(V, ld, n, j, w, sh.c, false, true, 1.0, sh);
+  int passes = 0, dependent = 0;
+  double nrm = 0.0;
+  for (;;) {
+    // sh.c holds the dot of a new pass
+    double sum = 0.0;
+    for (int i = 0; i < j; ++i) {
+      const double c = sh.c[i];
+      h[i] += c;
+      sum += c * c;
     }
-    __syncthreads();
-    double nrm;
-    if (sh.flag[0]) {
-      cta_dots<T>(V, ld, n, j, 1, w, sh);  // explicit norm
-      nrm = sqrt(sh.c[0]);
-    } else {
-      nrm = sqrt(sh.scal[1]);
-    }
+    const double self = sh.c[j];
+    if (self < 0.0) *err = 1;
+    const double onrm = sqrt(self < 0.0 ? 0.0 : self);
+    const double est = onrm * onrm - sum;  // the Pythagorean estimate of the new norm (bvorthog.c:124-127)
     ++passes;
-    if (threadIdx.x == 0) {
-      const double onrm = sh.scal[0];
-      sh.scal[2] = nrm;
-      sh.flag[1] = (passes < 3 && nrm != 0.0 && fabs(nrm) < eta * fabs(onrm));
-      sh.flag[3] = !(nrm != 0.0 && fabs(nrm) >= eta * fabs(onrm));
+    const bool estimated = est > 0.0;
+    if (!estimated) {
+      cta_sweep<T>(V, ld, n, j, w, sh.c, true, true, 1.0, sh);
+      const double s2 = sh.c[j];
+      nrm = sqrt(s2 < 0.0 ? 0.0 : s2);  // explicit norm
+    } else {
+      nrm = sqrt(est);
     }
-    __syncthreads();
-    more = sh.flag[1];
-    __syncthreads();
+    const bool more = passes < 3 && nrm != 0.0 && fabs(nrm) < eta * fabs(onrm);
+    dependent = !(nrm != 0.0 && fabs(nrm) >= eta * fabs(onrm));
+    if (more) {
+      if (estimated) cta_sweep<T>(V, ld, n, j, w, sh.c, true, true, 1.0, sh);
+      continue;
+    }
+    const double scale = nrm != 1.0 && nrm != 0.0 ? 1.0 / nrm : 1.0;
+    if (estimated) cta_sweep<T>(V, ld, n, j, w, sh.c, true, false, scale, sh);
+    else if (scale != 1.0) {
+      cta_scale<T>(w, n, scale);
+      if (threadIdx.x == 0) sh.bytes += 16ull * n;
+    }
+    break;
   }
-  const double nrm = sh.scal[2];
-  *lindep = sh.flag[3];
-  if (sh.flag[2]) *err = 1;
+  *lindep = dependent;
   *norm = nrm;
-  __syncthreads();
-  if (nrm != 1.0 && nrm != 0.0) {
-    cta_scale<T>(w, n, 1.0 / nrm);
-    if (threadIdx.x == 0) sh.bytes += 16ull * n;
-  }
+}
+
+// hypot: the plain square root where neither square can overflow or lose the sum to underflow (the QL
+// iteration is one chain of these)
+__device__ __forceinline__ double bhypot(double f, double g) {
+  const double q = fma(f, f, g * g);
+  return q > 1e-280 && q < 1e280 ? sqrt(q) : hypot(f, g);
 }
 
 // plane rotation [c s; -s c] [f; g] = [r; 0] with r carrying the sign of f
@@ -248,7 +310,7 @@ __device__ __forceinline__ void givens(double f, double g, double *c, double *s,
     *s = (g > 0.0) ? 1.0 : -1.0;
     *r = fabs(g);
   } else {
-    const double dd = hypot(f, g);
+    const double dd = bhypot(f, g);
     *c = fabs(f) / dd;
     *r = copysign(dd, f);
     *s = g / *r;
@@ -332,7 +394,7 @@ __device__ void ds_solve(BDs &ds, double *d, double *e, double *Q, double *wr, i
       for (; i >= L; --i) {
         double f = s * ee[i];
         const double b = c * ee[i];
-        r = hypot(f, g);
+        r = bhypot(f, g);
         ee[i + 1] = r;
         if (r == 0.0) {
           dd[i + 1] -= p;
