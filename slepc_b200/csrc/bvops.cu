@@ -183,7 +183,6 @@ __global__ void __launch_bounds__(kGemmThreads) panel_dmma_kernel(const TI *X, i
 // prefetches read other panels, and the only rows two CTAs touch at once are a box's extra rows past
 // its panel, whose values are never used.  Waits are bounded; a timeout sets g_panel_err and the CTA
 // stops (panel_gemm_error reads it).
-constexpr int kTmaThreads = kGemmThreads + 32;
 __device__ int g_panel_err;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -203,8 +202,8 @@ __device__ __forceinline__ bool mbar_wait_parity(uint64_t *bar, uint32_t parity)
 // The MMAs are the larger FP64 shapes (mma.sync.m16n8k16 .f64; m16n8k8 with KM = 8): 9% faster than
 // m8n8k4 on the 128^3 restart (fewer fragment loads per flop; the shapes share one peak) with the
 // same result bits.  TMA box of 68 rows: a column stride of 4 mod 16 doubles keeps every fragment
-// load of a half warp on distinct banks.  Eight consumer warps as four 16-row strips times two
-// halves of the 8-column tiles of Q.  Per KM-deep step a warp loads its A fragment once (KM/2
+// load of a half warp on distinct banks.  The consumer warps are four 16-row strips times NG
+// groups of the 8-column tiles of Q.  Per KM-deep step a warp loads its A fragment once (KM/2
 // doubles a lane) and reuses it across its tiles; Q's stride is also 4 mod 16.  Fragments
 // (g = lane / 4, t = lane % 4): A element i at row g + 8 (i % 2), depth t + 4 (i / 2); B element i
 // at depth t + 4 i, column g; D element i at row g + 8 (i / 2), column 2 t + i % 2.
@@ -228,8 +227,8 @@ __device__ __forceinline__ void dmma_16x8(double (&d)[4], const double (&a)[KM /
   }
 }
 
-template <int NT, int KM>
-__global__ void __launch_bounds__(kTmaThreads, 1) panel_dmma16_kernel(const __grid_constant__ CUtensorMap tx, double *Y,
+template <int NT, int KM, int NG>
+__global__ void __launch_bounds__(128 * NG + 32, 1) panel_dmma16_kernel(const __grid_constant__ CUtensorMap tx, double *Y,
                                                                       int ldy, int n, int kq,
                                                                       const double *__restrict__ Q, int ldq, int nc,
                                                                       double alpha, double beta, int stages) {
@@ -238,7 +237,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1) panel_dmma16_kernel(const __gr
   __shared__ __align__(8) uint64_t full[8], empty[8];
   __shared__ int last_issue[8];
   __shared__ volatile int stop;
-  constexpr int NTW = (NT + 1) / 2;  // 8-column tiles per consumer warp
+  constexpr int kTmaThreads = 128 * NG + 32;
+  constexpr int NTW = (NT + NG - 1) / NG;  // 8-column tiles per consumer warp
   constexpr int ncp = NT * 8;
   const int kp = (kq + KM - 1) / KM * KM;
   const int SQ = dmma16_q_stride(ncp);
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) panel_dmma16_kernel(const __gr
   if (tid == 0) {
     for (int s = 0; s < stages; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&full[s])), "r"(1) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&empty[s])), "r"(kGemmThreads / 32)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&empty[s])), "r"(4 * NG)
                    : "memory");
       last_issue[s] = -1;
     }
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) panel_dmma16_kernel(const __gr
   }
   __syncthreads();
   const uint32_t stage_bytes = (uint32_t)(stage_elems * sizeof(double));
-  if (warp == kGemmThreads / 32) {
+  if (warp == 4 * NG) {
     if (lane == 0) {
       for (int i = 0; i < mine && !stop; ++i) {
         const int s = i % stages;
@@ -291,6 +291,18 @@ __global__ void __launch_bounds__(kTmaThreads, 1) panel_dmma16_kernel(const __gr
     const int j0 = half * NTW, j1 = (half + 1) * NTW < NT ? (half + 1) * NTW : NT;
     for (int i = 0; i < mine && !stop; ++i) {
       const int s = i % stages;
+      const long long rb = (long long)(blockIdx.x + i * gridDim.x) * kRB + strip * 16 + g;
+      double yv[NTW][4];  // the previous values of Y travel while the panel lands and is multiplied
+      if (beta != 0.0) {
+#pragma unroll
+        for (int jj = 0; jj < NTW; ++jj)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const long long r = rb + 8 * (e / 2);
+            const int c = 8 * (j0 + jj) + 2 * t + (e % 2);
+            yv[jj][e] = j0 + jj < j1 && r < n && c < nc ? Y[(size_t)c * ldy + r] : 0.0;
+          }
+      }
       if (!mbar_wait_parity(&full[s], (i / stages) & 1)) {
         atomicOr(&g_panel_err, kDevErrTimeout);
         stop = 1;
@@ -318,7 +330,6 @@ __global__ void __launch_bounds__(kTmaThreads, 1) panel_dmma16_kernel(const __gr
       __syncwarp();
       if (lane == 0)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&empty[s])) : "memory");
-      const long long rb = (long long)(blockIdx.x + i * gridDim.x) * kRB + strip * 16 + g;
 #pragma unroll
       for (int jj = 0; jj < NTW; ++jj) {
         const int j = j0 + jj;
@@ -329,7 +340,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1) panel_dmma16_kernel(const __gr
             const int c = 8 * j + 2 * t + (e % 2);
             if (r < n && c < nc) {
               double *y = Y + (size_t)c * ldy + r;
-              *y = beta == 0.0 ? alpha * acc[jj][e] : alpha * acc[jj][e] + beta * *y;
+              *y = beta == 0.0 ? alpha * acc[jj][e] : alpha * acc[jj][e] + beta * yv[jj][e];
             }
           }
         }
@@ -868,6 +879,12 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // The pipelined FP64 product when X is FP64, 16-byte aligned with an even leading dimension, and two
 // or more stages fit in shared memory beside Q; cudaErrorNotSupported otherwise (the caller falls back).
+// Several CTAs per SM where three stages each fit: n = 262,144, 48 -> 16 columns 56 us with one, 43.5 with two,
+// 42.7 with three (92 before Y's values were loaded ahead of the product); wider products fit one and keep it.
+// 16 consumer warps instead of 8 from four 8-column tiles of Q on: the restart of n = 2,097,152, 80 -> 56 columns
+// 758 -> 711 us (26.4 TFLOP/s), n = 200,003, 40 -> 25 columns 51.1 -> 46.9; with two tiles 8 warps stay ahead (42.7 against 53.1 us).
+constexpr int kPanelCtas = 3;
+constexpr int kWideTiles = 4;
 template <int KM>
 cudaError_t panel_dmma16_launch(const double *X, int ldx, double *Y, int ldy, int n, int kq, const double *Q, int ldq,
                                 int nc, cudaStream_t stream, double alpha, double beta) {
@@ -877,7 +894,10 @@ cudaError_t panel_dmma16_launch(const double *X, int ldx, double *Y, int ldy, in
   const size_t qbytes = sizeof(double) * (size_t)kp * dmma16_q_stride(ncp);
   const size_t avail = max_dynamic_smem() - 1024 - 128;
   if (avail < qbytes + 2 * stage) return cudaErrorNotSupported;
-  int stages = (int)((avail - qbytes) / stage);
+  // narrow products leave room for several CTAs per SM, whose epilogues overlap: three stages each
+  int ctas = (int)((max_dynamic_smem() + 1024) / (qbytes + 3 * stage + 128 + 2048));
+  ctas = ctas < 1 ? 1 : ctas > kPanelCtas ? kPanelCtas : ctas;
+  int stages = ctas > 1 ? 3 : (int)((avail - qbytes) / stage);
   if (stages > 8) stages = 8;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return cudaErrorNotSupported;
@@ -892,17 +912,20 @@ cudaError_t panel_dmma16_launch(const double *X, int ldx, double *Y, int ldy, in
     return cudaErrorNotSupported;
   const size_t smem = qbytes + (size_t)stages * stage + 128;
   const int npanels = (n + kRB - 1) / kRB;
-  int grid = num_sms();
+  int grid = num_sms() * ctas;
   if (grid > npanels) grid = npanels;
   cudaError_t err = cudaSuccess;
   switch (nt) {
 #define B200_M16_CASE(NT)                                                                                          \
-  case NT:                                                                                                         \
-    err = cudaFuncSetAttribute(panel_dmma16_kernel<NT, KM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+  case NT: {                                                                                                       \
+    constexpr int NG = NT >= kWideTiles ? 4 : 2;                                                                   \
+    err = cudaFuncSetAttribute(panel_dmma16_kernel<NT, KM, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+                               (int)smem);                                                                         \
     if (err != cudaSuccess) return err;                                                                            \
-    panel_dmma16_kernel<NT, KM><<<grid, kTmaThreads, smem, stream>>>(tm, Y, ldy, n, kq, Q, ldq, nc, alpha, beta,      \
-                                                                     stages);                                      \
-    break;
+    panel_dmma16_kernel<NT, KM, NG><<<grid, 128 * NG + 32, smem, stream>>>(tm, Y, ldy, n, kq, Q, ldq, nc, alpha,   \
+                                                                           beta, stages);                          \
+    break;                                                                                                         \
+  }
     B200_M16_CASE(1) B200_M16_CASE(2) B200_M16_CASE(3) B200_M16_CASE(4) B200_M16_CASE(5) B200_M16_CASE(6)
     B200_M16_CASE(7) B200_M16_CASE(8) B200_M16_CASE(9) B200_M16_CASE(10) B200_M16_CASE(11) B200_M16_CASE(12)
     B200_M16_CASE(13) B200_M16_CASE(14) B200_M16_CASE(15) B200_M16_CASE(16)
