@@ -404,15 +404,16 @@ __device__ __forceinline__ void dmma_m16n8k16(double (&d)[4], const double (&a)[
 // Gram block M = Y^T X on the FP64 MMA path (mma.sync.m16n8k16.f64; tcgen05 has no FP64 kind), up to 64 columns of
 // each side per CTA (blockIdx.y, blockIdx.z select the 64-column blocks of Y and X).  The CTA's rows stream
 // through a ring of kGramStages stages of 32 rows with asynchronous copies (column stride 36 doubles, 4 mod 16: the
-// fragment loads of a half warp hit distinct banks).  The 8 warps are 16-column strips of Y (STRIPS) times the two
-// 16-row halves of a stage times, where warps are left, halves of X's 8-column tiles; the row halves meet in
-// shared memory at the end.  SELF: X is Y, staged once.  Fragments (g = lane / 4, t = lane % 4): A = Y^T, element e
+// fragment loads of a half warp hit distinct banks).  Warps 0..3 take the first 16 rows of a stage and warps 4..7 the
+// others, each a quarter of the products of the 16-column strips of Y (STRIPS) with the 8-column tiles of X, so that
+// the four schedulers have the same share; the row halves meet in shared memory at the end.  SELF: X is Y, staged once.  Fragments (g = lane / 4, t = lane % 4): A = Y^T, element e
 // at row g + 8 (e % 2), depth t + 4 (e / 2); B element e at depth t + 4 e, column g; D element e at row
 // g + 8 (e / 2), column 2 t + e % 2.  partial[cta * nx ny + i + j ny].
 //
 // Bound: for 48 x 48 columns of n = 262,144 rows 201 MB (31 us) and 1.2 GFLOP (33 us at the 37 TFLOP/s of this
-// shape).  A whole b200_bv_dot of that size takes 110 us with its read-back, 148 us with a CUDA-core kernel of register
-// tiles, which was bound by its shared-memory reads.
+// shape).  A whole b200_bv_dot of that size takes 97 us with its read-back (110 us with a strip per warp, which leaves
+// two warps idle at 48 columns), 148 us with a CUDA-core kernel of register tiles, which was bound by its
+// shared-memory reads.  Stages of 64 rows, or two or four of 32, make no difference.
 constexpr int kGramRows = 32;    // rows per stage
 constexpr int kGramLd = 36;      // doubles per staged column
 constexpr int kGramStages = 3;
@@ -421,16 +422,14 @@ __global__ void __launch_bounds__(256) gram_mma_kernel(const double *__restrict_
                                                        const double *__restrict__ Y, int ldy, int ny, int n,
                                                        double *partial) {
   extern __shared__ __align__(16) double gsm[];
-  constexpr int NH = STRIPS <= 2 ? 2 : 1;   // halves of X's column tiles
-  constexpr int TILES = 8 / NH;             // 8-column tiles of X a warp holds
+  constexpr int UNITS = 2 * STRIPS;  // most (strip, tile) products of a warp: a quarter of STRIPS x 8
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int y0 = blockIdx.y * 64, x0 = blockIdx.z * 64;
   const int cy = min(16 * STRIPS, ny - y0), cx = min(64, nx - x0);
   const int cyp = 16 * STRIPS, cxp = SELF ? 0 : (cx + 7) & ~7;  // staged columns (zero past cy, cx)
   const int stage = (cyp + cxp) * kGramLd;
-  const int strip = warp % STRIPS, kg = warp / STRIPS % 2, nh = warp / (2 * STRIPS);
-  const bool active = nh < NH;
-  const int tiles = (cx + 7) / 8, j0 = nh * ((tiles + NH - 1) / NH), j1 = min(tiles, j0 + (tiles + NH - 1) / NH);
+  const int kg = warp >> 2, tiles = (cx + 7) / 8, units = STRIPS * tiles;
+  const int u0 = (warp & 3) * units / 4, u1 = ((warp & 3) + 1) * units / 4, strip0 = u0 / tiles, tile0 = u0 - strip0 * tiles;
   const long long rows_per = ((long long)(n + gridDim.x - 1) / gridDim.x + kGramRows - 1) / kGramRows * kGramRows;
   const long long r0 = (long long)blockIdx.x * rows_per, r1 = min((long long)n, r0 + rows_per);
   const int nst = r1 > r0 ? (int)((r1 - r0 + kGramRows - 1) / kGramRows) : 0;
@@ -454,51 +453,62 @@ __global__ void __launch_bounds__(256) gram_mma_kernel(const double *__restrict_
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  double acc[TILES][4];
+  double acc[UNITS][4];
 #pragma unroll
-  for (int j = 0; j < TILES; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
+  for (int i = 0; i < UNITS; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0;
 #pragma unroll
   for (int st = 0; st < kGramStages - 1; ++st) load(st);
   for (int st = 0; st < nst; ++st) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kGramStages - 2) : "memory");
     __syncthreads();  // stage st has landed, stage st - 1 is consumed
     load(st + kGramStages - 1);
-    if (active) {
-      const double *ys = gsm + st % kGramStages * stage, *xs = SELF ? ys : ys + cyp * kGramLd;
-      const int k0 = 16 * kg;
-      double a[8];
+    const double *ys = gsm + st % kGramStages * stage + 16 * kg, *xs = SELF ? ys : ys + cyp * kGramLd;
+    double a[8];
+    int strip = strip0, tile = tile0;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) a[e] = ys[(16 * strip + g + 8 * (e & 1)) * kGramLd + k0 + t + 4 * (e >> 1)];
+    for (int i = 0; i < UNITS; ++i) {
+      if (u0 + i < u1) {
+        if (i == 0 || tile == 0)
 #pragma unroll
-      for (int j = 0; j < TILES; ++j) {
-        if (j0 + j < j1) {
-          double b[4];
+          for (int e = 0; e < 8; ++e) a[e] = ys[(16 * strip + g + 8 * (e & 1)) * kGramLd + t + 4 * (e >> 1)];
+        double b[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) b[e] = xs[(8 * (j0 + j) + g) * kGramLd + k0 + t + 4 * e];
-          dmma_m16n8k16(acc[j], a, b);
+        for (int e = 0; e < 4; ++e) b[e] = xs[(8 * tile + g) * kGramLd + t + 4 * e];
+        dmma_m16n8k16(acc[i], a, b);
+        if (++tile == tiles) {
+          tile = 0;
+          ++strip;
         }
       }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  // the second row half's sums through shared memory, [strip, half][element][lane]
-  double *other = gsm + (size_t)(strip * NH + (active ? nh : 0)) * TILES * 4 * 32 + lane;
-  if (active && kg == 1)
+  // the second row half's sums through shared memory, [warp][element][lane]
+  double *other = gsm + (size_t)(warp & 3) * UNITS * 4 * 32 + lane;
+  if (kg == 1)
 #pragma unroll
-    for (int j = 0; j < TILES; ++j)
+    for (int i = 0; i < UNITS; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) other[(j * 4 + e) * 32] = acc[j][e];
+      for (int e = 0; e < 4; ++e) other[(i * 4 + e) * 32] = acc[i][e];
   __syncthreads();
-  if (!active || kg != 0) return;
+  if (kg != 0) return;
   double *out = partial + (size_t)blockIdx.x * nx * ny;
+  int strip = strip0, tile = tile0;
 #pragma unroll
-  for (int j = 0; j < TILES; ++j)
+  for (int q = 0; q < UNITS; ++q) {
+    if (u0 + q < u1) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 16 * strip + g + 8 * (e >> 1), col = 8 * (j0 + j) + 2 * t + (e & 1);
-      if (j0 + j < j1 && i < cy && col < cx) out[(y0 + i) + (size_t)(x0 + col) * ny] = acc[j][e] + other[(j * 4 + e) * 32];
+      for (int e = 0; e < 4; ++e) {
+        const int i = 16 * strip + g + 8 * (e >> 1), col = 8 * tile + 2 * t + (e & 1);
+        if (i < cy && col < cx) out[(y0 + i) + (size_t)(x0 + col) * ny] = acc[q][e] + other[(q * 4 + e) * 32];
+      }
+      if (++tile == tiles) {
+        tile = 0;
+        ++strip;
+      }
     }
+  }
 }
 
 // The Gram pair on the FP64 MMA path (mma.sync.m16n8k16.f64), nc <= 64 columns: per 32-row chunk
@@ -582,23 +592,33 @@ __global__ void __launch_bounds__(256) gram_dual_mma_kernel(const double *__rest
 }
 
 // M(i, j) = the sum over the row blocks of the partial sums.  A CTA takes 32 consecutive pairs (one
-// per lane, so each load of a row block's partials is one coalesced 256-byte line); its 8 warps split
-// the row blocks (warp g sums blocks g, g + 8, ...) and the 8 sums are added in a fixed order.
-__global__ void __launch_bounds__(256) dot_final_kernel(const double *__restrict__ partial, int nblocks, int nx,
-                                                        int ny, double *M, int ldm) {
-  __shared__ double red[8][33];
+// per lane, so each load of a row block's partials is one coalesced 256-byte line); its 16 warps split
+// the row blocks (warp g sums blocks g, g + 16, ..., eight loads in flight) and their sums are added in a
+// fixed order.  Bound: latency (296 row blocks: 19 us with 8 warps and one load in flight each).
+constexpr int kFinalWarps = 16;
+__global__ void __launch_bounds__(32 * kFinalWarps) dot_final_kernel(const double *__restrict__ partial, int nblocks,
+                                                                     int nx, int ny, double *M, int ldm) {
+  __shared__ double red[kFinalWarps][33];
   const int npairs = nx * ny;
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int pr = blockIdx.x * 32 + lane;
   double acc = 0.0;
-  if (pr < npairs)
-    for (int b = g; b < nblocks; b += 8) acc += partial[(size_t)b * npairs + pr];
+  for (int b0 = g; b0 < nblocks; b0 += 8 * kFinalWarps) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int b = b0 + u * kFinalWarps;
+      v[u] = pr < npairs && b < nblocks ? __ldcg(partial + (size_t)b * npairs + pr) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc += v[u];
+  }
   red[g][lane] = acc;
   __syncthreads();
   if (g == 0 && pr < npairs) {
     double t = red[0][lane];
 #pragma unroll
-    for (int q = 1; q < 8; ++q) t += red[q][lane];
+    for (int q = 1; q < kFinalWarps; ++q) t += red[q][lane];
     M[(pr % ny) + (size_t)(pr / ny) * ldm] = t;
   }
 }
@@ -1147,7 +1167,7 @@ cudaError_t dot_launch(const double *X, int ldx, int nx, const double *Y, int ld
     dot_partial_kernel<<<blocks, 256, 0, stream>>>(X, ldx, nx, Y, ldy, ny, n, work);
   }
   count_launch();
-  dot_final_kernel<<<(npairs + 31) / 32, 256, 0, stream>>>(work, blocks, nx, ny, M, ldm);
+  dot_final_kernel<<<(npairs + 31) / 32, 32 * kFinalWarps, 0, stream>>>(work, blocks, nx, ny, M, ldm);
   count_launch();
   return cudaGetLastError();
 }
@@ -1168,7 +1188,7 @@ cudaError_t dot_dual_launch(const double *X, int ldx, const double *Y, int ldy, 
     default: gram_dual_mma_kernel<4><<<blocks, 256, 0, stream>>>(X, ldx, Y, ldy, nc, n, work); break;
   }
   count_launch();
-  dot_final_kernel<<<(npairs2 + 31) / 32, 256, 0, stream>>>(work, blocks, 2 * nc, nc, M, nc);
+  dot_final_kernel<<<(npairs2 + 31) / 32, 32 * kFinalWarps, 0, stream>>>(work, blocks, 2 * nc, nc, M, nc);
   count_launch();
   return cudaGetLastError();
 }
