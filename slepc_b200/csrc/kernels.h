@@ -59,6 +59,8 @@ struct SpmvTiles {
   int3 *longrows = nullptr;
   int nlong = 0;
   double *partials = nullptr;
+  int *seg_row = nullptr;      // index into longrows of each segment
+  unsigned *count = nullptr;   // segments of a long row that have finished, 0 between products
 };
 // Sliced ELL with 32-row slices for rows of at most kSellMaxRow nonzeros; the other rows go to
 // warp tiles and segments (rest).

@@ -168,6 +168,8 @@ static void part_free(CsrPart &P) {
   dev_free(P.wt.segs);
   dev_free(P.wt.longrows);
   dev_free(P.wt.partials);
+  dev_free(P.wt.seg_row);
+  dev_free(P.wt.count);
   dev_free(P.sell.off);
   dev_free(P.sell.width);
   dev_free(P.sell.mask);
@@ -177,6 +179,8 @@ static void part_free(CsrPart &P) {
   dev_free(P.sell.rest.segs);
   dev_free(P.sell.rest.longrows);
   dev_free(P.sell.rest.partials);
+  dev_free(P.sell.rest.seg_row);
+  dev_free(P.sell.rest.count);
   dev_free(P.sell.rest_rows);
   dev_free(P.sell.vals32);
   dev_free(P.vals32);
@@ -214,6 +218,34 @@ static b200_status part_upload(CsrPart &P, const int *rowptr, const int *colind,
   return B200_OK;
 }
 
+// Device copy of a plan of warp tiles and segments.  Returns with the copies done.
+static b200_status tiles_upload(SpmvTiles &T, const WarpTiles &wt, cudaStream_t s) {
+  T.ntiles = (int)wt.tiles.size();
+  T.nsegs = (int)wt.segs.size();
+  T.nlong = (int)wt.longrows.size();
+  if (T.ntiles) {
+    B200_CUDA_CHECK(dev_malloc(&T.tiles, sizeof(int4) * wt.tiles.size()));
+    B200_CUDA_CHECK(cudaMemcpyAsync(T.tiles, wt.tiles.data(), sizeof(int4) * wt.tiles.size(), cudaMemcpyHostToDevice, s));
+  }
+  std::vector<int> seg_row(wt.segs.size());
+  if (T.nsegs) {
+    for (int i = 0; i < T.nlong; ++i)
+      for (int k = 0; k < wt.longrows[i].z; ++k) seg_row[wt.longrows[i].y + k] = i;
+    B200_CUDA_CHECK(dev_malloc(&T.segs, sizeof(int2) * wt.segs.size()));
+    B200_CUDA_CHECK(dev_malloc(&T.partials, sizeof(double) * wt.segs.size()));
+    B200_CUDA_CHECK(dev_malloc(&T.longrows, sizeof(int3) * wt.longrows.size()));
+    B200_CUDA_CHECK(dev_malloc(&T.seg_row, sizeof(int) * seg_row.size()));
+    B200_CUDA_CHECK(dev_malloc(&T.count, sizeof(unsigned) * wt.longrows.size()));
+    B200_CUDA_CHECK(cudaMemsetAsync(T.count, 0, sizeof(unsigned) * wt.longrows.size(), s));
+    B200_CUDA_CHECK(cudaMemcpyAsync(T.segs, wt.segs.data(), sizeof(int2) * wt.segs.size(), cudaMemcpyHostToDevice, s));
+    B200_CUDA_CHECK(cudaMemcpyAsync(T.longrows, wt.longrows.data(), sizeof(int3) * wt.longrows.size(),
+                                    cudaMemcpyHostToDevice, s));
+    B200_CUDA_CHECK(cudaMemcpyAsync(T.seg_row, seg_row.data(), sizeof(int) * seg_row.size(), cudaMemcpyHostToDevice, s));
+  }
+  B200_CUDA_CHECK(cudaStreamSynchronize(s));
+  return B200_OK;
+}
+
 static b200_status part_build_sell(CsrPart &P, const int *rowptr_host, cudaStream_t s);
 
 // Row blocks (FP64 only), warp tiles and the sliced-ELL copy (the default schedule) from a host
@@ -226,23 +258,7 @@ static b200_status part_set_schedules(CsrPart &P, const int *rowptr_host, cudaSt
     B200_CUDA_CHECK(cudaMemcpyAsync(P.blocks, b.data(), sizeof(int) * b.size(), cudaMemcpyHostToDevice, s));
   }
   WarpTiles wt = spmv_warp_tiles(P.rows, rowptr_host);
-  P.wt.ntiles = (int)wt.tiles.size();
-  P.wt.nsegs = (int)wt.segs.size();
-  P.wt.nlong = (int)wt.longrows.size();
-  if (P.wt.ntiles) {
-    B200_CUDA_CHECK(dev_malloc(&P.wt.tiles, sizeof(int4) * wt.tiles.size()));
-    B200_CUDA_CHECK(
-        cudaMemcpyAsync(P.wt.tiles, wt.tiles.data(), sizeof(int4) * wt.tiles.size(), cudaMemcpyHostToDevice, s));
-  }
-  if (P.wt.nsegs) {
-    B200_CUDA_CHECK(dev_malloc(&P.wt.segs, sizeof(int2) * wt.segs.size()));
-    B200_CUDA_CHECK(dev_malloc(&P.wt.partials, sizeof(double) * wt.segs.size()));
-    B200_CUDA_CHECK(dev_malloc(&P.wt.longrows, sizeof(int3) * wt.longrows.size()));
-    B200_CUDA_CHECK(
-        cudaMemcpyAsync(P.wt.segs, wt.segs.data(), sizeof(int2) * wt.segs.size(), cudaMemcpyHostToDevice, s));
-    B200_CUDA_CHECK(cudaMemcpyAsync(P.wt.longrows, wt.longrows.data(), sizeof(int3) * wt.longrows.size(),
-                                    cudaMemcpyHostToDevice, s));
-  }
+  B200_CHECK(tiles_upload(P.wt, wt, s));
   B200_CUDA_CHECK(cudaStreamSynchronize(s));
   return part_build_sell(P, rowptr_host, s);
 }
@@ -281,24 +297,7 @@ static b200_status part_build_sell(CsrPart &P, const int *rowptr_host, cudaStrea
     B200_CUDA_CHECK(cudaMemcpyAsync(S.rest_rows, sp.rest_rows.data(), sizeof(int) * sp.rest_rows.size(),
                                     cudaMemcpyHostToDevice, s));
   }
-  WarpTiles &wt = sp.rest;
-  S.rest.ntiles = (int)wt.tiles.size();
-  S.rest.nsegs = (int)wt.segs.size();
-  S.rest.nlong = (int)wt.longrows.size();
-  if (S.rest.ntiles) {
-    B200_CUDA_CHECK(dev_malloc(&S.rest.tiles, sizeof(int4) * wt.tiles.size()));
-    B200_CUDA_CHECK(
-        cudaMemcpyAsync(S.rest.tiles, wt.tiles.data(), sizeof(int4) * wt.tiles.size(), cudaMemcpyHostToDevice, s));
-  }
-  if (S.rest.nsegs) {
-    B200_CUDA_CHECK(dev_malloc(&S.rest.segs, sizeof(int2) * wt.segs.size()));
-    B200_CUDA_CHECK(dev_malloc(&S.rest.partials, sizeof(double) * wt.segs.size()));
-    B200_CUDA_CHECK(dev_malloc(&S.rest.longrows, sizeof(int3) * wt.longrows.size()));
-    B200_CUDA_CHECK(
-        cudaMemcpyAsync(S.rest.segs, wt.segs.data(), sizeof(int2) * wt.segs.size(), cudaMemcpyHostToDevice, s));
-    B200_CUDA_CHECK(cudaMemcpyAsync(S.rest.longrows, wt.longrows.data(), sizeof(int3) * wt.longrows.size(),
-                                    cudaMemcpyHostToDevice, s));
-  }
+  B200_CHECK(tiles_upload(S.rest, sp.rest, s));
   B200_CUDA_CHECK(cudaStreamSynchronize(s));
   P.sell_ready = true;
   return B200_OK;

@@ -86,6 +86,37 @@ __global__ void __launch_bounds__(kSpmvThreads) spmv_rowblock_kernel(const int *
   }
 }
 
+// Tile {r0, r1, p0, p1} by one warp: prod holds kWarpTileNnz doubles of the warp's own.
+template <typename VT, typename XT>
+__device__ __forceinline__ void tile_rows(int4 tile, int lane, const int *__restrict__ rowptr,
+                                          const int *__restrict__ colind, const VT *__restrict__ vals,
+                                          const XT *__restrict__ x, double *__restrict__ y, double *prod) {
+  const int r0 = tile.x, nrows = tile.y - tile.x, p0 = tile.z, p1 = tile.w, cnt = p1 - p0;
+  const int myrow_start = (lane < nrows) ? __ldg(rowptr + r0 + lane) : 0;
+  const int next = __shfl_down_sync(0xffffffffu, myrow_start, 1);
+  const int myrow_end = (lane + 1 < nrows) ? next : p1;
+  VT a[kWarpTileNnz / 32];
+  int c[kWarpTileNnz / 32];
+#pragma unroll
+  for (int u = 0; u < kWarpTileNnz / 32; ++u) {
+    const int q = lane + 32 * u;
+    a[u] = (q < cnt) ? __ldcs(vals + p0 + q) : VT(0);
+    c[u] = (q < cnt) ? __ldcs(colind + p0 + q) : 0;
+  }
+#pragma unroll
+  for (int u = 0; u < kWarpTileNnz / 32; ++u) {
+    const int q = lane + 32 * u;
+    if (q < cnt) prod[q] = __dmul_rn((double)a[u], (double)__ldg(x + c[u]));
+  }
+  __syncwarp();
+  if (lane < nrows) {
+    double sacc = 0.0;
+    for (int q = myrow_start - p0; q < myrow_end - p0; ++q) sacc = __dadd_rn(sacc, prod[q]);
+    y[r0 + lane] = sacc;
+  }
+  __syncwarp();
+}
+
 // Warp tiles.  A tile {r0, r1, p0, p1} is <= 32 rows and <= kWarpTileNnz nonzeros; lane i of the owning
 // warp streams nonzeros i, i+32, ... (kWarpTileNnz/32 value, index and x loads in flight per
 // lane), keeps the rounded products in warp-private shared memory, and after a __syncwarp sums
@@ -106,35 +137,7 @@ __global__ void __launch_bounds__(kSpmvThreads) spmv_warptile_kernel(int ntiles,
   double *prod = prod_all[wib];
   const int nwarps = gridDim.x * (kSpmvThreads / 32);
   for (int t = blockIdx.x * (kSpmvThreads / 32) + wib; t < ntiles; t += nwarps) {
-    const int4 tile = tiles[t];
-    const int r0 = tile.x, r1 = tile.y, p0 = tile.z, p1 = tile.w;
-    const int nrows = r1 - r0;  // 1..32
-    const int cnt = p1 - p0;
-    // the nonzero range comes with the tile, so the value and index loads below do not wait
-    // for the row pointer; the row boundaries are needed only for the sums
-    const int myrow_start = (lane < nrows) ? __ldg(rowptr + r0 + lane) : 0;
-    const int next = __shfl_down_sync(0xffffffffu, myrow_start, 1);
-    const int myrow_end = (lane + 1 < nrows) ? next : p1;
-    VT a[kWarpTileNnz / 32];  // kept in the stored type until the multiply (fewer registers for FP32)
-    int c[kWarpTileNnz / 32];
-#pragma unroll
-    for (int u = 0; u < kWarpTileNnz / 32; ++u) {
-      const int q = lane + 32 * u;
-      a[u] = (q < cnt) ? __ldcs(vals + p0 + q) : VT(0);
-      c[u] = (q < cnt) ? __ldcs(colind + p0 + q) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < kWarpTileNnz / 32; ++u) {
-      const int q = lane + 32 * u;
-      if (q < cnt) prod[q] = __dmul_rn((double)a[u], (double)__ldg(x + c[u]));
-    }
-    __syncwarp();
-    if (lane < nrows) {
-      double sacc = 0.0;
-      for (int q = myrow_start - p0; q < myrow_end - p0; ++q) sacc = __dadd_rn(sacc, prod[q]);
-      y[r0 + lane] = sacc;
-    }
-    __syncwarp();
+    tile_rows(tiles[t], lane, rowptr, colind, vals, x, y, prod);
   }
 }
 
@@ -205,6 +208,27 @@ __global__ void __launch_bounds__(kSpmvThreads, sizeof(VT) == 4 ? 4 : 3)
   }
 }
 
+// Slice sl's row of this lane, in index order.
+template <typename VT, typename XT>
+__device__ __forceinline__ double slice_sum(long long base, int w, const VT *__restrict__ sval,
+                                            const int *__restrict__ scol, const XT *__restrict__ x) {
+  double sacc = 0.0;
+  for (int k0 = 0; k0 < w; k0 += 8) {
+    VT a[8];
+    int c[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const bool in = k0 + u < w;
+      c[u] = in ? __ldcs(scol + base + 32ll * (k0 + u)) : -1;
+      a[u] = in ? __ldcs(sval + base + 32ll * (k0 + u)) : VT(0);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (c[u] >= 0) sacc = __dadd_rn(sacc, __dmul_rn((double)a[u], (double)__ldg(x + c[u])));
+  }
+  return sacc;
+}
+
 // Sliced ELL (32-row slices): slice s stores its rows column-major in kSellWidth-padded chunks,
 // entry (row 32s+i, k) at off[s] + 32k + i, column -1 for padding; lane i of the owning warp sums
 // row 32s+i in index order (the same bits as a sequential CSR loop) with loads of 32 consecutive
@@ -226,103 +250,88 @@ __global__ void __launch_bounds__(kSpmvThreads) spmv_sell_kernel(int nslices, in
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * (kSpmvThreads / 32);
   for (int sl = blockIdx.x * (kSpmvThreads / 32) + (threadIdx.x >> 5); sl < nslices; sl += nwarps) {
-    const long long base = off[sl] + lane;
-    const int w = width[sl];
-    double sacc = 0.0;
-    for (int k0 = 0; k0 < w; k0 += 8) {
-      VT a[8];
-      int c[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const bool in = k0 + u < w;
-        c[u] = in ? __ldcs(scol + base + 32ll * (k0 + u)) : -1;
-        a[u] = in ? __ldcs(sval + base + 32ll * (k0 + u)) : VT(0);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (c[u] >= 0) sacc = __dadd_rn(sacc, __dmul_rn((double)a[u], (double)__ldg(x + c[u])));
-    }
+    const double sacc = slice_sum(off[sl] + lane, width[sl], sval, scol, x);
     const int r = 32 * sl + lane;
     if (r < n && ((mask[sl] >> lane) & 1u)) y[r] = sacc;
   }
 }
 
-// Segments of rows longer than a warp tile: segs[s] = {p_begin, p_end} (at most kSegmentNnz
-// nonzeros).  A warp streams its segment in chunks of kWarpTileNnz nonzeros with 8 independent
-// value/index loads and then 8 x gathers in flight per lane, adds each lane's products in a
-// fixed order, reduces the warp with a fixed shuffle tree and writes partials[s].  Half
-// occupancy buys the registers for the loads in flight; long dense-like rows (the power-law
-// columns of a transposed matrix) stream at full width.
+// Segment {p_begin, p_end} of a row longer than a warp tile (at most kSegmentNnz nonzeros): the warp
+// streams it in chunks of kWarpTileNnz nonzeros with 8 independent value/index loads and then 8 x
+// gathers in flight per lane, adds each lane's products in a fixed order and reduces the warp with a
+// fixed shuffle tree.
 template <typename VT, typename XT>
-__global__ void __launch_bounds__(kSpmvThreads, sizeof(VT) == 4 ? 4 : 3) spmv_segment_kernel(int nsegs, const int2 *__restrict__ segs,
-                                                                       const int *__restrict__ colind,
-                                                                       const VT *__restrict__ vals,
-                                                                       const XT *__restrict__ x,
-                                                                       double *__restrict__ partials,
-                                                                       const GsState *__restrict__ st, int step) {
-  if (st && st->halt && st->halt_step < step) return;
-  const int lane = threadIdx.x & 31;
-  const int nwarps = gridDim.x * (kSpmvThreads / 32);
-  for (int sg = blockIdx.x * (kSpmvThreads / 32) + (threadIdx.x >> 5); sg < nsegs; sg += nwarps) {
-    const int2 seg = segs[sg];
-    constexpr int U = kWarpTileNnz / 32;
-    double sacc = 0.0;
-    const int nfull = (seg.y - seg.x) / kWarpTileNnz;
+__device__ __forceinline__ double segment_sum(int2 seg, int lane, const int *__restrict__ colind,
+                                              const VT *__restrict__ vals, const XT *__restrict__ x) {
+  constexpr int U = kWarpTileNnz / 32;
+  double sacc = 0.0;
+  for (int p = seg.x + lane; p < seg.y + lane; p += kWarpTileNnz) {
     VT a[U];
     int c[U];
-    if (nfull > 0) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        a[u] = __ldcs(vals + seg.x + lane + 32 * u);
-        c[u] = __ldcs(colind + seg.x + lane + 32 * u);
-      }
+    for (int u = 0; u < U; ++u) {
+      const bool in = p + 32 * u < seg.y;
+      a[u] = in ? __ldcs(vals + p + 32 * u) : VT(0);
+      c[u] = in ? __ldcs(colind + p + 32 * u) : -1;
     }
-    // software pipeline: the values and indices of chunk k+1 are in flight while chunk k gathers x
-    for (int k = 0; k < nfull; ++k) {
-      double xv[U];
+    XT xv[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = (double)__ldg(x + c[u]);
-      VT an[U];
-      int cn[U];
-      if (k + 1 < nfull) {
-        const int pn = seg.x + (k + 1) * kWarpTileNnz + lane;
+    for (int u = 0; u < U; ++u) xv[u] = c[u] >= 0 ? __ldg(x + c[u]) : XT(0);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          an[u] = __ldcs(vals + pn + 32 * u);
-          cn[u] = __ldcs(colind + pn + 32 * u);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) sacc = __dadd_rn(sacc, __dmul_rn((double)a[u], xv[u]));
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        a[u] = an[u];
-        c[u] = cn[u];
-      }
-    }
-    const int p = seg.x + nfull * kWarpTileNnz;
-    for (int q = p + lane; q < seg.y; q += 32)
-      sacc = __dadd_rn(sacc, __dmul_rn((double)__ldcs(vals + q), (double)__ldg(x + __ldcs(colind + q))));
-    sacc = warp_sum(sacc);
-    if (lane == 0) partials[sg] = sacc;
+    for (int u = 0; u < U; ++u)
+      if (c[u] >= 0) sacc = __dadd_rn(sacc, __dmul_rn((double)a[u], (double)xv[u]));
   }
+  return warp_sum(sacc);
 }
 
-// y[row] of every long row from its segment partials: one warp per row, lane l adds partials
-// l, l+32, ... in order, then a fixed shuffle tree.  longrows[i] = {row, first slot, slot count}.
-__global__ void __launch_bounds__(256) spmv_fixup_kernel(int nlong, const int3 *__restrict__ longrows,
-                                                         const double *__restrict__ partials,
-                                                         double *__restrict__ y, const GsState *__restrict__ st,
-                                                         int step) {
+// A product whose rows are of mixed lengths in one launch: the segments of the longest rows first, then the
+// warp tiles, then the 32-row slices, one to a warp and dealt over the CTAs so that each has its share of every
+// kind.  The warp that finishes the last segment of a row (a count per row, which wraps to 0 for the next
+// product) adds the row's partial sums: lane l adds partials l, l + 32, ... in order, then a fixed shuffle tree.
+// Bound: latency of the index -> gather chains; a launch per kind leaves the chip to drain after each.
+// y = A x and z = A^T w of a 200,000 x 50,000 power-law matrix (4 million FP32 values; A is slices only) 42.2 us with
+// four launches for A^T, 22.4 us with one; FP64 values 47.1 -> 26.3.  Four CTAs per SM: five 22.8, six 23.7; loading
+// a segment's next chunk during the gathers takes 80 registers and 23.2 us (29.7 with FP64 values).
+template <typename VT, typename XT>
+__global__ void __launch_bounds__(kSpmvThreads, 4)
+    spmv_mixed_kernel(SpmvTiles T, const int *__restrict__ rowptr, const int *__restrict__ colind,
+                      const VT *__restrict__ vals, int nslices, int n, const long long *__restrict__ off,
+                      const int *__restrict__ width, const unsigned *__restrict__ mask, const VT *__restrict__ sval,
+                      const int *__restrict__ scol, const XT *__restrict__ x, double *__restrict__ y,
+                      const GsState *__restrict__ st, int step) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" :::);
   if (st && st->halt && st->halt_step < step) return;
-  const int lane = threadIdx.x & 31;
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= nlong) return;
-  const int3 lr = longrows[i];
-  double sacc = 0.0;
-  for (int k = lane; k < lr.z; k += 32) sacc += partials[lr.y + k];
-  sacc = warp_sum(sacc);
-  if (lane == 0) y[lr.x] = sacc;
+  __shared__ double prod[kSpmvThreads / 32][kWarpTileNnz];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int nwarps = gridDim.x * (kSpmvThreads / 32), total = T.nsegs + T.ntiles + nslices;
+  for (int it = wib * gridDim.x + blockIdx.x; it < total; it += nwarps) {
+    if (it < T.nsegs) {
+      const double s = segment_sum(T.segs[it], lane, colind, vals, x);
+      const int row = T.seg_row[it];
+      const int3 lr = T.longrows[row];
+      unsigned last = 0;
+      if (lane == 0) {
+        __stcg(T.partials + it, s);
+        __threadfence();
+        last = atomicInc(T.count + row, (unsigned)lr.z - 1) == (unsigned)lr.z - 1;
+        __threadfence();
+      }
+      if (__shfl_sync(0xffffffffu, last, 0)) {
+        double sacc = 0.0;
+        for (int k = lane; k < lr.z; k += 32) sacc += __ldcg(T.partials + lr.y + k);
+        sacc = warp_sum(sacc);
+        if (lane == 0) y[lr.x] = sacc;
+      }
+    } else if (it < T.nsegs + T.ntiles) {
+      tile_rows(T.tiles[it - T.nsegs], lane, rowptr, colind, vals, x, y, prod[wib]);
+    } else {
+      const int sl = it - T.nsegs - T.ntiles;
+      const double s = slice_sum(off[sl] + lane, width[sl], sval, scol, x);
+      const int r = 32 * sl + lane;
+      if (r < n && ((mask[sl] >> lane) & 1u)) y[r] = s;
+    }
+  }
 }
 
 template <int LPR>
@@ -450,30 +459,60 @@ WarpTiles spmv_warp_tiles(int n, const int *rowptr) {
 }
 
 template <typename VT, typename XT>
+cudaError_t spmv_mixed_launch(const SpmvTiles &T, const int *rowptr, const int *colind, const VT *vals,
+                              const SpmvSell &S, const VT *svals, int n, const XT *x, double *y, cudaStream_t stream,
+                              const GsState *st, int step) {
+  static int sms = 0, per_sm = 0;
+  if (!sms) {
+    int dev = 0, count = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmv_mixed_kernel<VT, XT>, kSpmvThreads, 0);
+    if (per_sm <= 0) per_sm = 1;
+    sms = count > 0 ? count : 1;
+  }
+  const int warps_per_cta = kSpmvThreads / 32, total = T.nsegs + T.ntiles + S.nslices;
+  int grid = (total + warps_per_cta - 1) / warps_per_cta;
+  if (grid > sms * per_sm) grid = sms * per_sm;  // persistent: every CTA resident at once
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kSpmvThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, spmv_mixed_kernel<VT, XT>, T, rowptr, colind, vals, S.nslices, n,
+                                           (const long long *)S.off, (const int *)S.width, (const unsigned *)S.mask,
+                                           svals, (const int *)S.cols, x, y, st, step);
+  if (e == cudaSuccess) count_launch();
+  return e;
+}
+
+template <typename VT, typename XT>
 cudaError_t spmv_warptile_launch_t(const SpmvTiles &T, const int *rowptr, const int *colind, const VT *vals,
                                    const XT *x, double *y, cudaStream_t stream, const GsState *st, int step,
                                    bool pipelined) {
-  static int sms = 0, tile_per_sm = 0, seg_per_sm = 0, pipe_per_sm = 0;
+  static int sms = 0, tile_per_sm = 0, pipe_per_sm = 0;
   if (!sms) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms <= 0) sms = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tile_per_sm, spmv_warptile_kernel<VT, XT>, kSpmvThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&seg_per_sm, spmv_segment_kernel<VT, XT>, kSpmvThreads, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pipe_per_sm, spmv_warptile_pipelined_kernel<VT, XT>, kSpmvThreads, 0);
     if (tile_per_sm <= 0) tile_per_sm = 1;
-    if (seg_per_sm <= 0) seg_per_sm = 1;
     if (pipe_per_sm <= 0) pipe_per_sm = 1;
   }
   const int warps_per_cta = kSpmvThreads / 32;
   // persistent grids: every CTA resident at once
   if (T.nsegs > 0) {
-    int grid = (T.nsegs + warps_per_cta - 1) / warps_per_cta;
-    if (grid > sms * seg_per_sm) grid = sms * seg_per_sm;
-    spmv_segment_kernel<VT, XT><<<grid, kSpmvThreads, 0, stream>>>(T.nsegs, T.segs, colind, vals, x, T.partials, st,
-                                                               step);
-    count_launch();
+    SpmvTiles segs = T;
+    segs.ntiles = 0;
+    const cudaError_t e =
+        spmv_mixed_launch<VT, XT>(segs, rowptr, colind, vals, SpmvSell{}, nullptr, 0, x, y, stream, st, step);
+    if (e != cudaSuccess) return e;
   }
   if (T.ntiles > 0) {
     int grid = (T.ntiles + warps_per_cta - 1) / warps_per_cta;
@@ -486,10 +525,6 @@ cudaError_t spmv_warptile_launch_t(const SpmvTiles &T, const int *rowptr, const 
       spmv_warptile_kernel<VT, XT><<<grid, kSpmvThreads, 0, stream>>>(T.ntiles, T.tiles, rowptr, colind, vals, x, y,
                                                                   st, step);
     }
-    count_launch();
-  }
-  if (T.nlong > 0) {
-    spmv_fixup_kernel<<<(T.nlong * 32 + 255) / 256, 256, 0, stream>>>(T.nlong, T.longrows, T.partials, y, st, step);
     count_launch();
   }
   return cudaGetLastError();
@@ -545,6 +580,8 @@ cudaError_t spmv_sell_launch_t(const SpmvSell &S, const VT *svals, int n, const 
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmv_sell_kernel<VT, XT>, kSpmvThreads, 0);
     if (per_sm <= 0) per_sm = 1;
   }
+  if (rest.ntiles > 0 || rest.nsegs > 0)
+    return spmv_mixed_launch<VT, XT>(rest, rowptr, colind, vals, S, svals, n, x, y, stream, st, step);
   if (S.nslices > 0) {
     int grid = (S.nslices + kSpmvThreads / 32 - 1) / (kSpmvThreads / 32);
     if (grid > sms * per_sm) grid = sms * per_sm;
@@ -562,10 +599,6 @@ cudaError_t spmv_sell_launch_t(const SpmvSell &S, const VT *svals, int n, const 
                                        y, st, step);
     if (e != cudaSuccess) return e;
     count_launch();
-  }
-  if (rest.ntiles > 0 || rest.nsegs > 0) {
-    cudaError_t e = spmv_warptile_launch_t<VT, XT>(rest, rowptr, colind, vals, x, y, stream, st, step, false);
-    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
