@@ -54,6 +54,7 @@ struct b200_neural_op_s {
   float *bias_part = nullptr;      // blocks' partial sums of the bias gradients
   float *mode_work = nullptr;      // modes_kernel: the blocks' shares and arrival counts
   unsigned *mode_count = nullptr;
+  float *grad_part = nullptr;      // blocks' partial sums of the weight gradients
   float2 *loss_part = nullptr, *loss_coef = nullptr;
   float *hloss = nullptr;    // pinned: B x K losses, then the error word
   cudaEvent_t loss_ready = nullptr;
@@ -226,18 +227,40 @@ long long bias_blocks(b200_neural_op op, int B) {
   return (long long)B * ((op->P + neural::kTile - 1) / neural::kTile);
 }
 
+// Weight gradient ma x mb of the one-pass form: columns of an output tile, tiles, and shares of the points (one
+// wave of blocks over all tiles).
+struct GradShape {
+  int cols, tiles, shares;
+};
+GradShape grad_shape(b200_neural_op op, int B, int ma, int mb) {
+  const int cols = mb <= 8 ? 8 : mb <= 16 ? 16 : 32;
+  const int tiles = ((ma + 31) / 32) * ((mb + cols - 1) / cols);
+  const long long chunks = (long long)B * ((op->P + neural::kGradPoints - 1) / neural::kGradPoints);
+  const long long fit = std::max(1, 148 * neural::kGradCtasPerSm / tiles);
+  return {cols, tiles, (int)std::min(fit, chunks)};
+}
+// The weight gradients of the network: W x 3, L of W x W, and for the output layers hidden x W and hidden x outputs.
+size_t grad_part_len(b200_neural_op op, int B) {
+  auto len = [&](int ma, int mb) {
+    const GradShape g = grad_shape(op, B, ma, mb);
+    return (size_t)g.tiles * g.shares * 32 * g.cols;
+  };
+  return len(op->W, 3) + op->L * len(op->W, op->W) + len(op->H, op->W) + len(op->H, op->K);
+}
+
 b200_status reserve(b200_neural_op op, int B) {
   if (B <= op->cap && op->act) return B200_OK;
   cudaFree(op->act);
   cudaFree(op->loss_bk);
   cudaFree(op->bias_part);
+  cudaFree(op->grad_part);
   cudaFree(op->loss_part);
   cudaFree(op->mode_work);
   cudaFree(op->mode_count);
   cudaFreeHost(op->hloss);
   op->act = nullptr;
   op->loss_bk = nullptr;
-  op->bias_part = op->mode_work = nullptr;
+  op->bias_part = op->grad_part = op->mode_work = nullptr;
   op->mode_count = nullptr;
   op->loss_part = op->loss_coef = nullptr;
   op->hloss = nullptr;
@@ -250,6 +273,7 @@ b200_status reserve(b200_neural_op op, int B) {
             cudaMallocHost(&op->hloss, sizeof(float) * BK + sizeof(int)) == cudaSuccess;
   if (ok && op->fused)
     ok = cudaMalloc(&op->bias_part, sizeof(float) * (size_t)bias_rows(op) * bias_blocks(op, B)) == cudaSuccess &&
+         cudaMalloc(&op->grad_part, sizeof(float) * grad_part_len(op, B)) == cudaSuccess &&
          cudaMalloc(&op->mode_work, sizeof(float) * (size_t)B * op->W * mode_blocks(op) * neural::kModeThreads) ==
              cudaSuccess &&
          cudaMalloc(&op->mode_count, sizeof(unsigned) * (size_t)B * op->W) == cudaSuccess &&
@@ -515,6 +539,27 @@ b200_status forward_fused(b200_neural_op op, int B, const float *feat, Acts &a, 
   return B200_OK;
 }
 
+// One weight gradient's partial sums, entered in the table for grad_final_kernel: C (ma x mb) = sum A B^T, C(i, j) at
+// grads[off + i * si + j * sj].
+cudaError_t grad_part(b200_neural_op op, int B, const float *A, int ma, const float *X, int mb, size_t off, int si, int sj,
+                      neural::GradTable &tab, int &blocks, long long &at) {
+  const GradShape g = grad_shape(op, B, ma, mb);
+  const int vec = op->P % 4 == 0 && (((uintptr_t)A | (uintptr_t)X) & 15) == 0;
+  const dim3 grid(g.tiles, g.shares);
+  const size_t smem = neural::grad_smem(g.cols / 8);
+  float *part = op->grad_part + at;
+  switch (g.cols) {
+    case 8: neural::grad_kernel<1><<<grid, neural::kGradThreads, smem, op->stream>>>(A, ma, X, mb, B, op->P, vec, part); break;
+    case 16: neural::grad_kernel<2><<<grid, neural::kGradThreads, smem, op->stream>>>(A, ma, X, mb, B, op->P, vec, part); break;
+    default: neural::grad_kernel<4><<<grid, neural::kGradThreads, smem, op->stream>>>(A, ma, X, mb, B, op->P, vec, part); break;
+  }
+  count_launch();
+  tab.t[tab.count++] = {blocks, ma, mb, g.cols, g.shares, si, sj, at, (long long)off};
+  blocks += g.tiles * g.cols;
+  at += (long long)g.tiles * g.shares * 32 * g.cols;
+  return cudaGetLastError();
+}
+
 b200_status loss_fused(b200_neural_op op, int B, const float *targets, const float *Y) {
   const int slices = (op->P + neural::kLossSlice - 1) / neural::kLossSlice, BK = B * op->K;
   neural::loss_part_kernel<<<dim3(slices, op->K, B), 256, 0, op->stream>>>(Y, targets, op->K, op->P, op->loss_part);
@@ -553,8 +598,14 @@ b200_status backward_fused(b200_neural_op op, int B, const float *feat, const fl
       part_w);
   count_launch();
   B200_CUDA_CHECK(cudaGetLastError());
-  B200_CUDA_CHECK(mix_grad(op, B, K, H, a.dY, a.Hh, grd(op, op->oQ2)));
-  B200_CUDA_CHECK(mix_grad(op, B, H, W, a.dH, a.V + L * B * WP, grd(op, op->oQ1)));
+  neural::GradTable tab{};
+  int grad_blocks = 0;
+  long long grad_at = 0;
+  auto grad = [&](const float *A, int ma, const float *X, int mb, size_t off, int si, int sj) {
+    return grad_part(op, B, A, ma, X, mb, off, si, sj, tab, grad_blocks, grad_at);
+  };
+  B200_CUDA_CHECK(grad(a.Hh, H, a.dY, K, op->oQ2, 1, H));
+  B200_CUDA_CHECK(grad(a.dH, H, a.V + L * B * WP, W, op->oQ1, W, 1));
   neural::PwArgs g{};
   g.Ci = W;
   g.Co = W;
@@ -566,7 +617,7 @@ b200_status backward_fused(b200_neural_op op, int B, const float *feat, const fl
   g.wc = W;
   g.T2 = a.T2;
   for (int l = L - 1; l >= 0; --l) {
-    B200_CUDA_CHECK(mix_grad(op, B, W, W, dU, a.V + l * B * WP, grd(op, op->oW[l])));
+    B200_CUDA_CHECK(grad(dU, W, a.V + l * B * WP, W, op->oW[l], W, 1));
     B200_CUDA_CHECK(field_modes(op, B * W, dU, a.dDh));
     B200_CUDA_CHECK(mode_mix(op, B, prm(op, op->oR[l]), a.dDh, a.T2, 1, a.Ch + l * B * W * M2, grd(op, op->oR[l])));
     g.X = dU;
@@ -577,7 +628,9 @@ b200_status backward_fused(b200_neural_op op, int B, const float *feat, const fl
     B200_CUDA_CHECK(pw(op, B, g));
     std::swap(dU, next);
   }
-  B200_CUDA_CHECK(mix_grad(op, B, W, 3, dU, feat, grd(op, op->oPw)));
+  B200_CUDA_CHECK(grad(dU, W, feat, 3, op->oPw, 3, 1));
+  neural::grad_final_kernel<<<grad_blocks, 256, 0, op->stream>>>(op->grad_part, tab, op->grads);
+  count_launch();
   neural::bias_rows_kernel<<<rows, 128, 0, op->stream>>>(op->bias_part, br, op->grads);
   count_launch();
   B200_CUDA_CHECK(cudaGetLastError());
@@ -629,7 +682,10 @@ extern "C" b200_status b200_neural_op_create(int N, int width, int modes, int la
             (!op->fused || (allow_max_dynamic_smem(neural::pw_kernel) == cudaSuccess &&
                             allow_max_dynamic_smem(neural::modes_kernel) == cudaSuccess &&
                             allow_max_dynamic_smem(neural::proj_fwd_kernel) == cudaSuccess &&
-                            allow_max_dynamic_smem(neural::proj_bwd_kernel) == cudaSuccess)) &&
+                            allow_max_dynamic_smem(neural::proj_bwd_kernel) == cudaSuccess &&
+                            allow_max_dynamic_smem(neural::grad_kernel<1>) == cudaSuccess &&
+                            allow_max_dynamic_smem(neural::grad_kernel<2>) == cudaSuccess &&
+                            allow_max_dynamic_smem(neural::grad_kernel<4>) == cudaSuccess)) &&
             cudaMalloc(&op->params, sizeof(float) * off) == cudaSuccess &&
             cudaMalloc(&op->grads, sizeof(float) * off) == cudaSuccess &&
             cudaMalloc(&op->adam_m, sizeof(float) * off) == cudaSuccess &&
@@ -672,6 +728,7 @@ extern "C" b200_status b200_neural_op_destroy(b200_neural_op op) {
   cudaFree(op->act);
   cudaFree(op->loss_bk);
   cudaFree(op->bias_part);
+  cudaFree(op->grad_part);
   cudaFree(op->loss_part);
   cudaFree(op->mode_work);
   cudaFree(op->mode_count);

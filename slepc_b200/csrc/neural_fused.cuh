@@ -4,11 +4,11 @@
 // 4 FP32 multiply-adds per byte that must move, so HBM bounds it and not the arithmetic.  These kernels
 // therefore do each step in one pass over the activations: channel mix, spectral term, bias, activation
 // (or its derivative) and the bias gradients' partial sums, in FP32 FMAs (packed two to an instruction,
-// fma.rn.f32x2) with the weights broadcast from shared memory.  The weight gradients, whose contraction
-// runs over the grid, stay tensor-core products (tcgemm.cu).
+// fma.rn.f32x2) with the weights broadcast from shared memory.  The weight gradients contract over the grid:
+// each reads its two fields once, and one kernel adds the blocks' sums of all of them.
 //
 // Measured (loss and gradients, width 32, 16 modes, 4 layers): 512 x 512 grid, batch 4, 12.2 ms as separate
-// products and elementwise kernels (113 launches), 4.4 ms so (44 launches); 64 x 64 grid, batch 16, 1.55 -> 0.96 ms.
+// products and elementwise kernels (113 launches), 3.8 ms so (38 launches); 64 x 64 grid, batch 16, 1.58 -> 0.91 ms.
 #pragma once
 #include "common.h"
 
@@ -675,6 +675,152 @@ __global__ void __launch_bounds__(128) bias_rows_kernel(const float *__restrict_
     __syncthreads();
   }
   if (threadIdx.x == 0) grads[r.off[t] + c] = red[0];
+}
+
+// Weight gradients C[i][j] = sum over the batch and the points of A[b][i][p] B[b][j][p].  A block takes 32 rows of A
+// and 8 NV of B over its share of the 64-point chunks (blockIdx.x: tile of the output, blockIdx.y: share), staged by
+// asynchronous copies in a ring of kGradStages chunks.  Each of the four warps takes 16 of the 64 points; lane
+// (gi, gj) = (lane / 8, lane % 8) holds rows gi + 4 u and columns gj + 8 v (rows 68 floats apart: the loads of four
+// points of eight rows hit distinct banks), even and odd points in the halves of packed FP32 FMAs.  The block's
+// sums go to part[tile][share][i][j]; grad_final_kernel adds the shares of every tensor in a fixed order.
+// Bound: HBM (32 x 32 over 4 x 512^2 points: 268 MB, 42 us) and FP32 FMAs (30 us).
+// Measured there 69 us, a split-depth tensor-core product with its own sum 165 (3-product TF32); 64 x 32 130 against
+// 294, 32 x 3 33 against 128; the sums of all seven gradients 10 us in one launch against 14 each.
+constexpr int kGradThreads = 128, kGradPoints = 64, kGradLd = kGradPoints + 4, kGradStages = 4, kGradCtasPerSm = 3;
+__host__ __device__ constexpr size_t grad_smem(int nv) {
+  return sizeof(float) * (size_t)kGradStages * (32 + 8 * nv) * kGradLd;
+}
+template <int NV>
+__global__ void __launch_bounds__(kGradThreads) grad_kernel(const float *__restrict__ A, int ma, const float *__restrict__ B,
+                                                          int mb, int batch, int P, int vec, float *part) {
+  extern __shared__ __align__(16) float gsm[];
+  constexpr int kRows = 32 + 8 * NV, kStage = kRows * kGradLd;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gi = lane >> 3, gj = lane & 7;
+  const int jt = (mb + 8 * NV - 1) / (8 * NV), i0 = blockIdx.x / jt * 32, j0 = blockIdx.x % jt * (8 * NV);
+  const int ra = min(32, ma - i0), rb = min(8 * NV, mb - j0);
+  const int per = (P + kGradPoints - 1) / kGradPoints;  // chunks of a field
+  const long long total = (long long)batch * per;
+  const long long c0 = total * blockIdx.y / gridDim.y, c1 = total * (blockIdx.y + 1) / gridDim.y;
+  const int n = (int)(c1 - c0);
+  for (int e = tid; e < kGradStages * kStage; e += kGradThreads) gsm[e] = 0.f;  // rows past ra, rb stay zero
+  __syncthreads();
+  int b = (int)(c0 / per), c = (int)(c0 - (long long)b * per);  // the next chunk to stage
+  auto load = [&](int st) {
+    if (st < n) {
+      const uint32_t d = (uint32_t)__cvta_generic_to_shared(gsm + st % kGradStages * kStage);
+      const int p0 = c * kGradPoints;
+      const float *a = A + ((size_t)b * ma + i0) * P + p0, *x = B + ((size_t)b * mb + j0) * P + p0;
+      if (vec) {
+#pragma unroll
+        for (int e = tid; e < kRows * (kGradPoints / 4); e += kGradThreads) {
+          const int r = e / (kGradPoints / 4), q = 4 * (e % (kGradPoints / 4)), rr = r < 32 ? r : r - 32;
+          if (rr < (r < 32 ? ra : rb)) {
+            const bool in = p0 + q < P;
+            const float *src = (r < 32 ? a : x) + (size_t)rr * P + (in ? q : 0);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + 4u * (uint32_t)(r * kGradLd + q)),
+                         "l"(src), "r"(in ? 16 : 0)
+                         : "memory");
+          }
+        }
+      } else {
+        for (int e = tid; e < kRows * kGradPoints; e += kGradThreads) {
+          const int r = e / kGradPoints, q = e % kGradPoints, rr = r < 32 ? r : r - 32;
+          if (rr < (r < 32 ? ra : rb)) {
+            const bool in = p0 + q < P;
+            const float *src = (r < 32 ? a : x) + (size_t)rr * P + (in ? q : 0);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4u * (uint32_t)(r * kGradLd + q)),
+                         "l"(src), "r"(in ? 4 : 0)
+                         : "memory");
+          }
+        }
+      }
+      if (++c == per) {
+        c = 0;
+        ++b;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned long long acc[8][NV];
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[u][v] = 0ull;
+#pragma unroll
+  for (int st = 0; st < kGradStages - 1; ++st) load(st);
+  for (int st = 0; st < n; ++st) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kGradStages - 2) : "memory");
+    __syncthreads();  // chunk st has landed, chunk st - 1 is consumed
+    load(st + kGradStages - 1);
+    const float *s = gsm + st % kGradStages * kStage + 16 * warp;
+#pragma unroll
+    for (int q = 0; q < 16; q += 4) {
+      ulonglong2 bv[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) bv[v] = *reinterpret_cast<const ulonglong2 *>(s + (32 + gj + 8 * v) * kGradLd + q);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const ulonglong2 av = *reinterpret_cast<const ulonglong2 *>(s + (gi + 4 * u) * kGradLd + q);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          fma2(acc[u][v], av.x, bv[v].x);
+          fma2(acc[u][v], av.y, bv[v].y);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  constexpr int kOut = 32 * 8 * NV;  // four warps' sums fit the ring: 4 kOut <= kGradStages kStage
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const float2 h = unpack2(acc[u][v]);
+      gsm[warp * kOut + (gi + 4 * u) * (8 * NV) + gj + 8 * v] = h.x + h.y;
+    }
+  __syncthreads();
+  float *out = part + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * kOut;
+  for (int e = tid; e < kOut; e += kGradThreads)
+    out[e] = (gsm[e] + gsm[kOut + e]) + (gsm[2 * kOut + e] + gsm[3 * kOut + e]);
+}
+
+// A tensor's partial sums: output (i, j) of tile t at part[at + ((t * shares + share) * 32 + i % 32) * cols + j % cols],
+// to grads[off + i * si + j * sj].
+struct GradTensor {
+  int first;          // first block of grad_final_kernel
+  int ma, mb, cols, shares, si, sj;
+  long long at, off;
+};
+struct GradTable {
+  int count;
+  GradTensor t[20];
+};
+// A block takes 32 consecutive outputs of a tile; its 8 warps every eighth share, eight loads in flight.
+__global__ void __launch_bounds__(256) grad_final_kernel(const float *__restrict__ part, const __grid_constant__ GradTable tab,
+                                                         float *grads) {
+  __shared__ float red[8][32];
+  int k = 0;
+  while (k + 1 < tab.count && (int)blockIdx.x >= tab.t[k + 1].first) ++k;
+  const GradTensor &t = tab.t[k];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, outs = 32 * t.cols;
+  const int e0 = (blockIdx.x - t.first) * 32 + lane, tile = e0 / outs, e = e0 - tile * outs;
+  const float *p = part + t.at + (size_t)tile * t.shares * outs + e;
+  float acc = 0.f;
+  for (int s0 = warp; s0 < t.shares; s0 += 64) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = s0 + 8 * u < t.shares ? __ldcg(p + (size_t)(s0 + 8 * u) * outs) : 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc += v[u];
+  }
+  red[warp][lane] = acc;
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) acc += red[w][lane];
+  const int jt = (t.mb + t.cols - 1) / t.cols, i = tile / jt * 32 + e / t.cols, j = tile % jt * t.cols + e % t.cols;
+  if (i < t.ma && j < t.mb) grads[t.off + (long long)i * t.si + (long long)j * t.sj] = acc;
 }
 
 }  // namespace neural
