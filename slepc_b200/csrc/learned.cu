@@ -531,7 +531,7 @@ b200_status forward_fused(b200_neural_op op, int B, const float *feat, Acts &a, 
     B200_CUDA_CHECK(pw(op, B, g));
   }
   const int Hp = (H + 31) & ~31;
-  const size_t smem = sizeof(float) * ((size_t)(W + 32) * neural::kTile + (size_t)W * Hp + (size_t)Hp * 16 + Hp);
+  const size_t smem = sizeof(float) * ((size_t)(W + 16) * neural::kTile + (size_t)W * Hp + (size_t)Hp * 16 + Hp);
   neural::proj_fwd_kernel<<<dim3((op->P + neural::kTile - 1) / neural::kTile, B), neural::kPwThreads, smem, op->stream>>>(
       a.V + L * B * WP, W, H, K, op->P, prm(op, op->oQ1), prm(op, op->oq1), prm(op, op->oQ2), prm(op, op->oq2), a.Z, a.Hh, Y);
   count_launch();
@@ -590,7 +590,7 @@ b200_status backward_fused(b200_neural_op op, int B, const float *feat, const fl
   };
   float *part_k = bias(K, op->oq2), *part_h = bias(H, op->oq1), *part_w = bias(W, op->ob[L - 1]);
   const int Hp = (H + 31) & ~31;
-  const size_t smem = sizeof(float) * ((size_t)(64 + K) * neural::kTile + (size_t)K * Hp + (size_t)Hp * 32);
+  const size_t smem = sizeof(float) * ((size_t)(32 + K) * neural::kTile + (size_t)K * Hp + (size_t)Hp * 32);
   float *dU = a.dV0, *next = a.dV1;  // dU holds the gradient before layer l's activation
   neural::proj_bwd_kernel<<<dim3((op->P + neural::kTile - 1) / neural::kTile, B, (W + 31) / 32),
                                 neural::kPwThreads, smem, op->stream>>>(

@@ -8,7 +8,7 @@
 // each reads its two fields once, and one kernel adds the blocks' sums of all of them.
 //
 // Measured (loss and gradients, width 32, 16 modes, 4 layers): 512 x 512 grid, batch 4, 12.2 ms as separate
-// products and elementwise kernels (113 launches), 3.8 ms so (38 launches); 64 x 64 grid, batch 16, 1.58 -> 0.91 ms.
+// products and elementwise kernels (113 launches), 3.6 ms so (38 launches); 64 x 64 grid, batch 16, 1.58 -> 0.84 ms.
 #pragma once
 #include "common.h"
 
@@ -79,15 +79,16 @@ __device__ __forceinline__ void mix16(Acc &acc, const float *X, const float *W, 
   }
 }
 
-// the 4 points x 16 outputs of a thread to its rows of a [16][kTile] tile
+// a thread's 4 points of its outputs O0..O1-1 to the rows of a [O1 - O0][kTile] tile
+template <int O0 = 0, int O1 = 16>
 __device__ __forceinline__ void acc_to_tile(const Acc &acc, float *tile, int t) {
 #pragma unroll
-  for (int o = 0; o < 16; o += 2)
+  for (int o = O0; o < O1; o += 2)
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const float2 f = unpack2(acc.v[u][o >> 1]);
-      tile[o * kTile + t + 64 * u] = f.x;
-      tile[(o + 1) * kTile + t + 64 * u] = f.y;
+      tile[(o - O0) * kTile + t + 64 * u] = f.x;
+      tile[(o + 1 - O0) * kTile + t + 64 * u] = f.y;
     }
 }
 
@@ -258,16 +259,17 @@ __global__ void __launch_bounds__(kPwThreads) pw_kernel(PwArgs a) {
 
 // Projection, forward: Z = Q1 V + q1, H = gelu(Z), Y = Q2 H + q2 (at most 16 outputs), 32 hidden channels at a
 // time (16 per half of the block; the halves' shares of Y meet at the end): V is read once, Z, H and Y are
-// written once.
-__global__ void __launch_bounds__(kPwThreads) proj_fwd_kernel(const float *__restrict__ V, int W, int H, int K, int P,
+// written once.  Z and H pass through shared memory 8 channels of a half at a time: three blocks fit an SM
+// (with proj_bwd_kernel's, loss and gradients of 512 x 512, batch 4 take 3.60 ms instead of 3.76).
+__global__ void __launch_bounds__(kPwThreads, 3) proj_fwd_kernel(const float *__restrict__ V, int W, int H, int K, int P,
                                                               const float *__restrict__ Q1, const float *__restrict__ q1,
                                                               const float *__restrict__ Q2, const float *__restrict__ q2,
                                                               float *Z, float *Hh, float *Y) {
   extern __shared__ __align__(16) float sm[];
   const int Hp = (H + 31) & ~31;
   float *Xs = sm;              // [W][kTile]
-  float *Hs = Xs + W * kTile;  // [32][kTile]: Z then H of the group; at the end the second half's share of Y
-  float *w1 = Hs + 32 * kTile; // [W][Hp]
+  float *Hs = Xs + W * kTile;  // [2][8][kTile]: Z then H of 8 channels per half; at the end the second half's share of Y
+  float *w1 = Hs + 16 * kTile; // [W][Hp]
   float *w2 = w1 + W * Hp;     // [Hp][16]
   float *b1 = w2 + Hp * 16;    // [Hp]
   const int tid = threadIdx.x, t = tid & 63, half = tid >> 6, b = blockIdx.y, p0 = blockIdx.x * kTile;
@@ -280,7 +282,7 @@ __global__ void __launch_bounds__(kPwThreads) proj_fwd_kernel(const float *__res
   __syncthreads();
   Acc y;
   y.zero();
-  float *mine = Hs + 16 * half * kTile;  // a thread reads and writes its own points of its half's channels only
+  float *mine = Hs + 8 * half * kTile;  // a thread reads and writes its own points of its half's channels only
   for (int h0 = 16 * half; h0 < Hp; h0 += 32) {
     Acc z;
 #pragma unroll
@@ -288,23 +290,27 @@ __global__ void __launch_bounds__(kPwThreads) proj_fwd_kernel(const float *__res
 #pragma unroll
       for (int u = 0; u < 4; ++u) z.v[u][o] = pack2(b1[h0 + 2 * o], b1[h0 + 2 * o + 1]);
     mix16(z, Xs, w1 + h0, Hp, W, t);
-    acc_to_tile(z, mine, t);
-    const int mh = min(16, H - h0);
-#pragma unroll 1
-    for (int h = 0; h < mh; ++h) {
-      const size_t at = ((size_t)b * H + h0 + h) * P + p0 + t;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float *z1 = mine + h * kTile + t + 64 * u;
-        const float x = *z1, g = gelu(x);
-        *z1 = g;
-        if (p0 + t + 64 * u < P) {
-          Z[at + 64 * u] = x;
-          Hh[at + 64 * u] = g;
+    for (int part = 0; part < 2; ++part) {
+      const int h8 = h0 + 8 * part, mh = min(8, H - h8);
+      if (part == 0) acc_to_tile<0, 8>(z, mine, t);
+      else acc_to_tile<8, 16>(z, mine, t);
+#pragma unroll 1
+      for (int h = 0; h < mh; ++h) {
+        const size_t at = ((size_t)b * H + h8 + h) * P + p0 + t;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float *z1 = mine + h * kTile + t + 64 * u;
+          const float x = *z1, g = gelu(x);
+          *z1 = g;
+          if (p0 + t + 64 * u < P) {
+            Z[at + 64 * u] = x;
+            Hh[at + 64 * u] = g;
+          }
         }
       }
+      mix16(y, mine, w2 + h8 * 16, 16, max(mh, 0), t);
     }
-    mix16(y, mine, w2 + h0 * 16, 16, max(mh, 0), t);
   }
   __syncthreads();
   if (half) acc_to_tile(y, Hs, t);
@@ -373,17 +379,17 @@ __global__ void loss_final_kernel(const float2 *__restrict__ part, int slices, i
 
 // Projection, backward: dY = cu T + cy Y (written for the gradient of Q2), dH = Q2^T dY, dZ = dH gelu'(Z)
 // (written for the gradient of Q1), dV = Q1^T dZ for at most 32 channels per blockIdx.z, and the partial sums of
-// dq2, dq1 (z = 0) and of dV.  Hidden channels go 32 at a time.
-__global__ void __launch_bounds__(kPwThreads) proj_bwd_kernel(const float *__restrict__ Y, const float *__restrict__ T,
+// dq2, dq1 (z = 0) and of dV.  Hidden channels go 32 at a time; gelu' replaces Z in place before dH is formed, so
+// that one tile serves all three and three blocks fit an SM.
+__global__ void __launch_bounds__(kPwThreads, 3) proj_bwd_kernel(const float *__restrict__ Y, const float *__restrict__ T,
                                                               const float2 *__restrict__ coef, const float *__restrict__ Z,
                                                               int W, int H, int K, int P, const float *__restrict__ Q1,
                                                               const float *__restrict__ Q2, float *dY, float *dZ,
                                                               float *dV, float *part_k, float *part_h, float *part_w) {
   extern __shared__ __align__(16) float sm[];
   const int Hp = (H + 31) & ~31, c0 = blockIdx.z * 32, nc = min(32, W - c0);
-  float *Zs = sm;                  // [32][kTile]: Z of the group, then dZ; at the end dV
-  float *Ds = Zs + 32 * kTile;     // [32][kTile]: dH of the group
-  float *Ys = Ds + 32 * kTile;     // [K][kTile]: dY
+  float *Zs = sm;                  // [32][kTile]: Z of the group, then gelu'(Z), then dZ; at the end dV
+  float *Ys = Zs + 32 * kTile;     // [K][kTile]: dY
   float *w2 = Ys + K * kTile;      // [K][Hp]
   float *w1 = w2 + K * Hp;         // [Hp][32]
   const int tid = threadIdx.x, t = tid & 63, half = tid >> 6, b = blockIdx.y, p0 = blockIdx.x * kTile;
@@ -411,27 +417,31 @@ __global__ void __launch_bounds__(kPwThreads) proj_bwd_kernel(const float *__res
   if (first) tile_sums(Ys, K, part_k + blk, blocks);
   Acc g;
   g.zero();
-  float *zh = Zs + 16 * half * kTile + t, *dh = Ds + 16 * half * kTile + t;
+  float *zh = Zs + 16 * half * kTile + t;
   for (int g0 = 0; g0 < H; g0 += 32) {
     stage_wait();
     __syncthreads();
     const int h0 = g0 + 16 * half, mh = min(16, H - h0);
+    // a thread's own points and channels: no barrier
+#pragma unroll 1
+    for (int h = 0; h < mh; ++h)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) zh[h * kTile + 64 * u] = gelu_grad(zh[h * kTile + 64 * u]);
     {
       Acc d;
       d.zero();
       mix16(d, Ys, w2 + h0, Hp, K, t);
-      acc_to_tile(d, Ds + 16 * half * kTile, t);
-    }
-    // a thread's own points and channels: no barrier
-#pragma unroll 1
-    for (int h = 0; h < mh; ++h) {
-      const size_t at = ((size_t)b * H + h0 + h) * P + p0 + t;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float x = dh[h * kTile + 64 * u] * gelu_grad(zh[h * kTile + 64 * u]);  // dY = 0 past P
-        zh[h * kTile + 64 * u] = x;
-        if (first && p0 + t + 64 * u < P) dZ[at + 64 * u] = x;
-      }
+      for (int h = 0; h < 16; ++h)
+        if (h < mh) {
+          const size_t at = ((size_t)b * H + h0 + h) * P + p0 + t;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float x = d.get(u, h) * zh[h * kTile + 64 * u];  // dY = 0 past P
+            zh[h * kTile + 64 * u] = x;
+            if (first && p0 + t + 64 * u < P) dZ[at + 64 * u] = x;
+          }
+        }
     }
     const int mg = min(32, H - g0);
     if (first) tile_sums(Zs, mg, part_h + (size_t)g0 * blocks + blk, blocks);
@@ -613,7 +623,7 @@ __global__ void __launch_bounds__(256) mode_mix_kernel(const float *__restrict__
     x %= W;
     float acc = 0.f;
     if (q < M2) {
-#pragma unroll 8
+#pragma unroll 16
       for (int y = 0; y < W; ++y)
         acc = fmaf(__ldg(R + ((size_t)(transposed ? y * W + x : x * W + y)) * M2 + q),
                    __ldg(in + ((size_t)b * W + y) * M2 + q), acc);
@@ -626,6 +636,7 @@ __global__ void __launch_bounds__(256) mode_mix_kernel(const float *__restrict__
       float d[kModes];
 #pragma unroll
       for (int k = 0; k < kModes; ++k) d[k] = k < M ? D[k * M + m] : 0.f;
+#pragma unroll 4
       for (int i = q >> 4; i < N; i += 16) {
         const float4 *s = reinterpret_cast<const float4 *>(Sp + (size_t)i * kModes);
         float t = 0.f;
