@@ -54,12 +54,11 @@ WarpTiles spmv_warp_tiles(int n, const int *rowptr_host);
 struct SpmvTiles {
   int4 *tiles = nullptr;
   int ntiles = 0;
-  int2 *segs = nullptr;
+  int4 *segs = nullptr;        // {p_begin, p_end, index into longrows, segments of that row}
   int nsegs = 0;
   int3 *longrows = nullptr;
   int nlong = 0;
   double *partials = nullptr;
-  int *seg_row = nullptr;      // index into longrows of each segment
   unsigned *count = nullptr;   // segments of a long row that have finished, 0 between products
 };
 // Sliced ELL with 32-row slices for rows of at most kSellMaxRow nonzeros; the other rows go to

@@ -168,7 +168,6 @@ static void part_free(CsrPart &P) {
   dev_free(P.wt.segs);
   dev_free(P.wt.longrows);
   dev_free(P.wt.partials);
-  dev_free(P.wt.seg_row);
   dev_free(P.wt.count);
   dev_free(P.sell.off);
   dev_free(P.sell.width);
@@ -179,7 +178,6 @@ static void part_free(CsrPart &P) {
   dev_free(P.sell.rest.segs);
   dev_free(P.sell.rest.longrows);
   dev_free(P.sell.rest.partials);
-  dev_free(P.sell.rest.seg_row);
   dev_free(P.sell.rest.count);
   dev_free(P.sell.rest_rows);
   dev_free(P.sell.vals32);
@@ -227,20 +225,21 @@ static b200_status tiles_upload(SpmvTiles &T, const WarpTiles &wt, cudaStream_t 
     B200_CUDA_CHECK(dev_malloc(&T.tiles, sizeof(int4) * wt.tiles.size()));
     B200_CUDA_CHECK(cudaMemcpyAsync(T.tiles, wt.tiles.data(), sizeof(int4) * wt.tiles.size(), cudaMemcpyHostToDevice, s));
   }
-  std::vector<int> seg_row(wt.segs.size());
+  std::vector<int4> segs;
   if (T.nsegs) {
     for (int i = 0; i < T.nlong; ++i)
-      for (int k = 0; k < wt.longrows[i].z; ++k) seg_row[wt.longrows[i].y + k] = i;
-    B200_CUDA_CHECK(dev_malloc(&T.segs, sizeof(int2) * wt.segs.size()));
+      for (int k = 0; k < wt.longrows[i].z; ++k) {
+        const int2 p = wt.segs[wt.longrows[i].y + k];
+        segs.push_back({p.x, p.y, i, wt.longrows[i].z});
+      }
+    B200_CUDA_CHECK(dev_malloc(&T.segs, sizeof(int4) * wt.segs.size()));
     B200_CUDA_CHECK(dev_malloc(&T.partials, sizeof(double) * wt.segs.size()));
     B200_CUDA_CHECK(dev_malloc(&T.longrows, sizeof(int3) * wt.longrows.size()));
-    B200_CUDA_CHECK(dev_malloc(&T.seg_row, sizeof(int) * seg_row.size()));
     B200_CUDA_CHECK(dev_malloc(&T.count, sizeof(unsigned) * wt.longrows.size()));
     B200_CUDA_CHECK(cudaMemsetAsync(T.count, 0, sizeof(unsigned) * wt.longrows.size(), s));
-    B200_CUDA_CHECK(cudaMemcpyAsync(T.segs, wt.segs.data(), sizeof(int2) * wt.segs.size(), cudaMemcpyHostToDevice, s));
+    B200_CUDA_CHECK(cudaMemcpyAsync(T.segs, segs.data(), sizeof(int4) * segs.size(), cudaMemcpyHostToDevice, s));
     B200_CUDA_CHECK(cudaMemcpyAsync(T.longrows, wt.longrows.data(), sizeof(int3) * wt.longrows.size(),
                                     cudaMemcpyHostToDevice, s));
-    B200_CUDA_CHECK(cudaMemcpyAsync(T.seg_row, seg_row.data(), sizeof(int) * seg_row.size(), cudaMemcpyHostToDevice, s));
   }
   B200_CUDA_CHECK(cudaStreamSynchronize(s));
   return B200_OK;

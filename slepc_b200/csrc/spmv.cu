@@ -288,10 +288,11 @@ __device__ __forceinline__ double segment_sum(int2 seg, int lane, const int *__r
 // warp tiles, then the 32-row slices, one to a warp and dealt over the CTAs so that each has its share of every
 // kind.  The warp that finishes the last segment of a row (a count per row, which wraps to 0 for the next
 // product) adds the row's partial sums: lane l adds partials l, l + 32, ... in order, then a fixed shuffle tree.
+// With T.count null the partial sums stay for spmv_fixup_kernel.
 // Bound: latency of the index -> gather chains; a launch per kind leaves the chip to drain after each.
 // y = A x and z = A^T w of a 200,000 x 50,000 power-law matrix (4 million FP32 values; A is slices only) 42.2 us with
-// four launches for A^T, 22.4 us with one; FP64 values 47.1 -> 26.3.  Four CTAs per SM: five 22.8, six 23.7; loading
-// a segment's next chunk during the gathers takes 80 registers and 23.2 us (29.7 with FP64 values).
+// four launches for A^T, 21.7 us with one; FP64 values 47.1 -> 26.  Four CTAs per SM: six 24; loading a segment's
+// next chunk during the gathers takes 80 registers and 24.3 us.
 template <typename VT, typename XT>
 __global__ void __launch_bounds__(kSpmvThreads, 4)
     spmv_mixed_kernel(SpmvTiles T, const int *__restrict__ rowptr, const int *__restrict__ colind,
@@ -307,19 +308,31 @@ __global__ void __launch_bounds__(kSpmvThreads, 4)
   const int nwarps = gridDim.x * (kSpmvThreads / 32), total = T.nsegs + T.ntiles + nslices;
   for (int it = wib * gridDim.x + blockIdx.x; it < total; it += nwarps) {
     if (it < T.nsegs) {
-      const double s = segment_sum(T.segs[it], lane, colind, vals, x);
-      const int row = T.seg_row[it];
-      const int3 lr = T.longrows[row];
+      const int4 seg = T.segs[it];
+      const double s = segment_sum(make_int2(seg.x, seg.y), lane, colind, vals, x);
       unsigned last = 0;
-      if (lane == 0) {
-        __stcg(T.partials + it, s);
-        __threadfence();
-        last = atomicInc(T.count + row, (unsigned)lr.z - 1) == (unsigned)lr.z - 1;
-        __threadfence();
+      if (lane == 0) __stcg(T.partials + it, s);
+      if (lane == 0 && T.count) {
+        const unsigned wrap = (unsigned)seg.w - 1;
+        unsigned before;
+        asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;"
+                     : "=r"(before)
+                     : "l"(T.count + seg.z), "r"(wrap)
+                     : "memory");
+        last = before == wrap;
       }
-      if (__shfl_sync(0xffffffffu, last, 0)) {
+      __syncwarp();
+      if (T.count && __shfl_sync(0xffffffffu, last, 0)) {
+        const int3 lr = T.longrows[seg.z];
         double sacc = 0.0;
-        for (int k = lane; k < lr.z; k += 32) sacc += __ldcg(T.partials + lr.y + k);
+        for (int k0 = lane; k0 < lr.z; k0 += 256) {
+          double v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) v[u] = k0 + 32 * u < lr.z ? __ldcg(T.partials + lr.y + k0 + 32 * u) : 0.0;
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (k0 + 32 * u < lr.z) sacc += v[u];
+        }
         sacc = warp_sum(sacc);
         if (lane == 0) y[lr.x] = sacc;
       }
@@ -332,6 +345,22 @@ __global__ void __launch_bounds__(kSpmvThreads, 4)
       if (r < n && ((mask[sl] >> lane) & 1u)) y[r] = s;
     }
   }
+}
+
+// y[row] of every long row from its segment partials, in the same order: one warp per row.
+__global__ void __launch_bounds__(256) spmv_fixup_kernel(int nlong, const int3 *__restrict__ longrows,
+                                                         const double *__restrict__ partials,
+                                                         double *__restrict__ y, const GsState *__restrict__ st,
+                                                         int step) {
+  if (st && st->halt && st->halt_step < step) return;
+  const int lane = threadIdx.x & 31;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= nlong) return;
+  const int3 lr = longrows[i];
+  double sacc = 0.0;
+  for (int k = lane; k < lr.z; k += 32) sacc += partials[lr.y + k];
+  sacc = warp_sum(sacc);
+  if (lane == 0) y[lr.x] = sacc;
 }
 
 template <int LPR>
@@ -483,11 +512,22 @@ cudaError_t spmv_mixed_launch(const SpmvTiles &T, const int *rowptr, const int *
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, spmv_mixed_kernel<VT, XT>, T, rowptr, colind, vals, S.nslices, n,
+  // A warp waits for a round trip to L2 after each of its segments when the rows' counts are kept.  With many
+  // segments to a warp a launch that adds the partial sums costs less: 200,000 x 50,000 (4 thousand segments) 21.7 us
+  // against 25.3 with it, 1,200,000 x 300,000 (24 thousand) 106 against 95, 2,000,000 x 500,000 177 against 150.
+  SpmvTiles U = T;
+  const bool fixup = T.nsegs > 2 * sms * per_sm * warps_per_cta;
+  if (fixup) U.count = nullptr;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, spmv_mixed_kernel<VT, XT>, U, rowptr, colind, vals, S.nslices, n,
                                            (const long long *)S.off, (const int *)S.width, (const unsigned *)S.mask,
                                            svals, (const int *)S.cols, x, y, st, step);
-  if (e == cudaSuccess) count_launch();
-  return e;
+  if (e != cudaSuccess) return e;
+  count_launch();
+  if (fixup) {
+    spmv_fixup_kernel<<<(T.nlong * 32 + 255) / 256, 256, 0, stream>>>(T.nlong, T.longrows, T.partials, y, st, step);
+    count_launch();
+  }
+  return cudaGetLastError();
 }
 
 template <typename VT, typename XT>

@@ -20,6 +20,26 @@ LENGTHS = {
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_many_segments(b200, dtype):
+    """More segments than two per resident warp: their sum is a launch of its own."""
+    import torch
+
+    rng = np.random.default_rng(3)
+    m, n = 23, 600001
+    rowptr = (np.arange(m + 1) * n).astype(np.int32)
+    vals = rng.standard_normal((m, n)).astype(dtype)
+    A = b200.Mat().createAIJ((rowptr, np.tile(np.arange(n, dtype=np.int32), m), vals.ravel()), size=(m, n), dtype=dtype)
+    V = vals.astype(np.float64)
+    for _ in range(2):
+        x = rng.standard_normal(n)
+        xd = torch.from_numpy(x).cuda()
+        yd = torch.full((m,), np.nan, dtype=torch.float64, device="cuda")
+        A.mult(xd.data_ptr(), yd.data_ptr())
+        torch.cuda.synchronize()
+        assert np.all(np.abs(yd.cpu().numpy() - V @ x) <= 2 * (n + 2) * 2.0 ** -53 * (np.abs(V) @ np.abs(x)))
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("name", sorted(LENGTHS))
 def test_mixed_rows(b200, name, dtype):
     import torch
