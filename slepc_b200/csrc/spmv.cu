@@ -511,13 +511,16 @@ cudaError_t spmv_mixed_launch(const SpmvTiles &T, const int *rowptr, const int *
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
   // A warp waits for a round trip to L2 after each of its segments when the rows' counts are kept.  With many
   // segments to a warp a launch that adds the partial sums costs less: 200,000 x 50,000 (4 thousand segments) 21.7 us
   // against 25.3 with it, 1,200,000 x 300,000 (24 thousand) 106 against 95, 2,000,000 x 500,000 177 against 150.
   SpmvTiles U = T;
   const bool fixup = T.nsegs > 2 * sms * per_sm * warps_per_cta;
   if (fixup) U.count = nullptr;
+  // Launched as a programmatic dependent where the launch counts (21.5 us against 23.4 for the small pair above); a
+  // large product before it keeps the SMs to itself, without waiting blocks and their shared memory beside its
+  // cache (a solve with the operator A^T A of the 2,000,000 x 500,000 matrix 29.2 ms against 34.4).
+  cfg.numAttrs = fixup ? 0 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, spmv_mixed_kernel<VT, XT>, U, rowptr, colind, vals, S.nslices, n,
                                            (const long long *)S.off, (const int *)S.width, (const unsigned *)S.mask,
                                            svals, (const int *)S.cols, x, y, st, step);
