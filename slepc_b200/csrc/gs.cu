@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, 1) gs_column_kernel(ColumnParams p, 
 // no divisions and give every warp one share.
 // Measured (BVMatLanczos on 2-D Laplacians, whole calls; column by column / one CTA per SM / one cluster):
 // n = 3,660 columns 0..30 583 / 356 / 232 us; n = 10,000 columns 16..32 373 / 221 / 195; n = 14,400 columns
-// 0..20 428 / 254 / 192; n = 40,000 columns 0..40 1,031 / 592 / -; n = 65,000 columns 0..20 508 / 320 / -.
+// 0..20 428 / 254 / 192; n = 40,000 columns 0..40 1,030 / 612 / -; n = 65,000 columns 0..20 508 / 319 / -.
 // So the cluster runs wherever its shared memory holds the basis, then one CTA per SM wherever that does.
 constexpr int kRunWarps = 16;
 constexpr int kRunThreads = kRunWarps * 32;
@@ -636,7 +636,8 @@ __global__ void __launch_bounds__(kRunThreads, 1) gs_run_kernel(RunParams p, con
   const int G = gridDim.x, n = p.n, spc = p.spc, R = 32 * spc;
   const int r0 = blockIdx.x * R, rows = min(R, n - r0);
   const int lp = 31 - __clz(kRunWarps / spc);  // parts of the columns in an update: 1 << lp warps to a slice
-  const int slice = warp % spc, part = warp / spc;
+  // a warp's slice and share of the columns; with lp = 0 it owns whole slices, and past spc none
+  const int slice = lp ? warp % spc : warp, part = lp ? warp / spc : 0;
   double *ws = run_smem;       // w of the CTA's rows
   double *ups = ws + R;        // partial updates [part][row]
   double *Vs = ups + (R << lp);  // basis columns [column][row]
