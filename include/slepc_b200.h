@@ -591,7 +591,9 @@ b200_status b200_neural_op_forward(b200_neural_op op, int batch, const float *fe
 /* mean loss against targets_dev (batch x nout x N*N) */
 b200_status b200_neural_op_loss(b200_neural_op op, int batch, const float *features_dev, const float *targets_dev,
                                 float *loss);
-/* loss and its gradient with respect to every parameter (grads_host nullable, nparams floats) */
+/* loss and its gradient with respect to every parameter (grads_host nullable, nparams floats).  features_dev and
+ * targets_dev may be refilled or freed as soon as this call or the next one returns, also where the backward pass
+ * is still running then (grads_host null) */
 b200_status b200_neural_op_loss_grad(b200_neural_op op, int batch, const float *features_dev,
                                      const float *targets_dev, float *loss, float *grads_host);
 /* one Adam step (beta1 0.9, beta2 0.999, eps 1e-8) on the loss of one batch */

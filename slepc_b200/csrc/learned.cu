@@ -560,18 +560,22 @@ cudaError_t grad_part(b200_neural_op op, int B, const float *A, int ma, const fl
   return cudaGetLastError();
 }
 
-b200_status loss_fused(b200_neural_op op, int B, const float *targets, const float *Y) {
+b200_status loss_fused(b200_neural_op op, int B, const float *targets, const Acts &a, bool want_grad) {
   const int slices = (op->P + neural::kLossSlice - 1) / neural::kLossSlice, BK = B * op->K;
-  neural::loss_part_kernel<<<dim3(slices, op->K, B), 256, 0, op->stream>>>(Y, targets, op->K, op->P, op->loss_part);
+  neural::loss_part_kernel<<<dim3(slices, op->K, B), 256, 0, op->stream>>>(a.Y, targets, op->K, op->P, op->loss_part);
   count_launch();
   neural::loss_final_kernel<<<(BK + 127) / 128, 128, 0, op->stream>>>(op->loss_part, slices, BK, 1.f / (float)BK, op->loss_bk,
                                                                      op->loss_coef);
   count_launch();
+  if (want_grad) {
+    neural::loss_grad_kernel<<<dim3(slices, op->K, B), 256, 0, op->stream>>>(a.Y, targets, op->loss_coef, op->K, op->P, a.dY);
+    count_launch();
+  }
   B200_CUDA_CHECK(cudaGetLastError());
   return loss_queue_read(op, B);
 }
 
-b200_status backward_fused(b200_neural_op op, int B, const float *feat, const float *targets, Acts &a) {
+b200_status backward_fused(b200_neural_op op, int B, const float *feat, Acts &a) {
   const int W = op->W, L = op->L, M = op->M, H = op->H, K = op->K;
   const size_t WP = (size_t)W * op->P, M2 = (size_t)M * M;
   // partial bias sums, tensor by tensor: rows of this tensor's blocks
@@ -594,8 +598,7 @@ b200_status backward_fused(b200_neural_op op, int B, const float *feat, const fl
   float *dU = a.dV0, *next = a.dV1;  // dU holds the gradient before layer l's activation
   neural::proj_bwd_kernel<<<dim3((op->P + neural::kTile - 1) / neural::kTile, B, (W + 31) / 32),
                                 neural::kPwThreads, smem, op->stream>>>(
-      a.Y, targets, op->loss_coef, a.Z, W, H, K, op->P, prm(op, op->oQ1), prm(op, op->oQ2), a.dY, a.dH, dU, part_k, part_h,
-      part_w);
+      a.dY, a.Z, W, H, K, op->P, prm(op, op->oQ1), prm(op, op->oQ2), a.dH, dU, part_k, part_h, part_w);
   count_launch();
   B200_CUDA_CHECK(cudaGetLastError());
   neural::GradTable tab{};
@@ -786,9 +789,17 @@ extern "C" b200_status b200_neural_op_loss_grad(b200_neural_op op, int batch, co
   size_t len;
   Acts a = carve(op, &len);
   if (op->fused) {
-    B200_CHECK(forward_fused(op, batch, features_dev, a, a.Y));
-    B200_CHECK(loss_fused(op, batch, targets_dev, a.Y));
-    B200_CHECK(backward_fused(op, batch, features_dev, targets_dev, a));
+    // Without a read-back the call returns while the backward pass runs: it reads a copy of the features then,
+    // and the caller's buffers are free on return.
+    const float *feat = features_dev;
+    if (!grads_host) {
+      B200_CUDA_CHECK(cudaMemcpyAsync(a.F, features_dev, sizeof(float) * (size_t)batch * 3 * op->P,
+                                      cudaMemcpyDeviceToDevice, op->stream));
+      feat = a.F;
+    }
+    B200_CHECK(forward_fused(op, batch, feat, a, a.Y));
+    B200_CHECK(loss_fused(op, batch, targets_dev, a, true));
+    B200_CHECK(backward_fused(op, batch, feat, a));
   } else {
     B200_CHECK(forward(op, batch, features_dev, a));
     B200_CHECK(loss(op, batch, targets_dev, a, true));
@@ -826,7 +837,7 @@ extern "C" b200_status b200_neural_op_loss(b200_neural_op op, int batch, const f
   Acts a = carve(op, &len);
   if (op->fused) {
     B200_CHECK(forward_fused(op, batch, features_dev, a, a.Y));
-    B200_CHECK(loss_fused(op, batch, targets_dev, a.Y));
+    B200_CHECK(loss_fused(op, batch, targets_dev, a, false));
   } else {
     B200_CHECK(forward(op, batch, features_dev, a));
     B200_CHECK(loss(op, batch, targets_dev, a, false));

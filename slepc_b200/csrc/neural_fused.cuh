@@ -377,15 +377,26 @@ __global__ void loss_final_kernel(const float2 *__restrict__ part, int slices, i
   coef[e] = make_float2(-2.f * yu / yy * scale, 2.f * yu * yu / (yy * yy) * scale);
 }
 
-// Projection, backward: dY = cu T + cy Y (written for the gradient of Q2), dH = Q2^T dY, dZ = dH gelu'(Z)
-// (written for the gradient of Q1), dV = Q1^T dZ for at most 32 channels per blockIdx.z, and the partial sums of
-// dq2, dq1 (z = 0) and of dV.  Hidden channels go 32 at a time; gelu' replaces Z in place before dH is formed, so
-// that one tile serves all three and three blocks fit an SM.
-__global__ void __launch_bounds__(kPwThreads, 3) proj_bwd_kernel(const float *__restrict__ Y, const float *__restrict__ T,
-                                                              const float2 *__restrict__ coef, const float *__restrict__ Z,
+// dY = cu T + cy Y over the slices of loss_part_kernel.  A kernel of its own, before the loss is read back, so that
+// no later kernel reads the caller's targets.
+__global__ void __launch_bounds__(256) loss_grad_kernel(const float *__restrict__ Y, const float *__restrict__ T,
+                                                        const float2 *__restrict__ coef, int K, int P, float *dY) {
+  const int k = blockIdx.y, b = blockIdx.z;
+  const size_t base = ((size_t)b * K + k) * P;
+  const float2 cf = __ldg(coef + b * K + k);
+  const int p1 = min(P, (int)(blockIdx.x + 1) * kLossSlice);
+#pragma unroll 4
+  for (int p = blockIdx.x * kLossSlice + threadIdx.x; p < p1; p += 256)
+    dY[base + p] = cf.x * __ldg(T + base + p) + cf.y * __ldg(Y + base + p);
+}
+
+// Projection, backward: dH = Q2^T dY, dZ = dH gelu'(Z) (written for the gradient of Q1), dV = Q1^T dZ for at most 32
+// channels per blockIdx.z, and the partial sums of dq2, dq1 (z = 0) and of dV.  Hidden channels go 32 at a time;
+// gelu' replaces Z in place before dH is formed, so that one tile serves all three and three blocks fit an SM.
+__global__ void __launch_bounds__(kPwThreads, 3) proj_bwd_kernel(const float *__restrict__ dY, const float *__restrict__ Z,
                                                               int W, int H, int K, int P, const float *__restrict__ Q1,
-                                                              const float *__restrict__ Q2, float *dY, float *dZ,
-                                                              float *dV, float *part_k, float *part_h, float *part_w) {
+                                                              const float *__restrict__ Q2, float *dZ, float *dV,
+                                                              float *part_k, float *part_h, float *part_w) {
   extern __shared__ __align__(16) float sm[];
   const int Hp = (H + 31) & ~31, c0 = blockIdx.z * 32, nc = min(32, W - c0);
   float *Zs = sm;                  // [32][kTile]: Z of the group, then gelu'(Z), then dZ; at the end dV
@@ -396,24 +407,12 @@ __global__ void __launch_bounds__(kPwThreads, 3) proj_bwd_kernel(const float *__
   const bool first = blockIdx.z == 0;
   const size_t blocks = (size_t)gridDim.x * gridDim.y, blk = (size_t)b * gridDim.x + blockIdx.x;
   stage_tile<kTile>(Zs, Z + (size_t)b * H * P, min(32, H), P, p0);
+  stage_tile<kTile>(Ys, dY + (size_t)b * K * P, K, P, p0);  // zero past P
   stage_commit();
   for (int e = tid; e < K * Hp; e += kPwThreads) w2[e] = e % Hp < H ? Q2[(e / Hp) * H + e % Hp] : 0.f;
   for (int e = tid; e < Hp * 32; e += kPwThreads)
     w1[e] = (e >> 5) < H && (e & 31) < nc ? Q1[(e >> 5) * W + c0 + (e & 31)] : 0.f;
-#pragma unroll 2
-  for (int k = half; k < K; k += 2) {
-    const float2 cf = __ldg(coef + b * K + k);
-    const size_t at = ((size_t)b * K + k) * P + p0 + t;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      float d = 0.f;
-      if (p0 + t + 64 * u < P) {
-        d = cf.x * __ldg(T + at + 64 * u) + cf.y * __ldg(Y + at + 64 * u);
-        if (first) dY[at + 64 * u] = d;
-      }
-      Ys[k * kTile + t + 64 * u] = d;
-    }
-  }
+  stage_wait();
   if (first) tile_sums(Ys, K, part_k + blk, blocks);
   Acc g;
   g.zero();
