@@ -183,7 +183,8 @@ using namespace b200;
 
 namespace {
 
-// Activation layout for batch cap: offsets (in floats) into op->act
+// Activation layout for batch cap: offsets (in floats) into op->act.  T1, Dh, dU and dCh serve the separate products
+// only: the one-pass form leaves them null, and with them the room that its partial sums take.
 struct Acts {
   float *F, *V, *U, *Ch, *T1, *Dh, *T2, *Z, *Hh, *Y;  // forward
   float *dY, *dH, *dV0, *dV1, *dU, *dDh, *dCh;        // backward
@@ -198,12 +199,13 @@ Acts carve(b200_neural_op op, size_t *len) {
     off += (n + 63) / 64 * 64;
     return p;
   };
+  auto separate = [&](size_t n) { return op->fused ? nullptr : take(n); };
   a.F = take(B * 3 * P);
   a.V = take((L + 1) * B * W * P);
   a.U = take(L * B * W * P);
   a.Ch = take(L * B * W * M2);
-  a.T1 = take(B * W * NM);
-  a.Dh = take(B * W * M2);
+  a.T1 = separate(B * W * NM);
+  a.Dh = separate(B * W * M2);
   a.T2 = take(B * W * NM);
   a.Z = take(B * op->H * P);
   a.Hh = take(B * op->H * P);
@@ -212,9 +214,9 @@ Acts carve(b200_neural_op op, size_t *len) {
   a.dH = take(B * op->H * P);
   a.dV0 = take(B * W * P);
   a.dV1 = take(B * W * P);
-  a.dU = take(B * W * P);
+  a.dU = separate(B * W * P);
   a.dDh = take(B * W * M2);
-  a.dCh = take(B * W * M2);
+  a.dCh = separate(B * W * M2);
   *len = off;
   return a;
 }
@@ -288,6 +290,7 @@ b200_status reserve(b200_neural_op op, int B) {
   }
   if (op->fused) op->loss_coef = op->loss_part + BK * slices;
   op->act_len = len;
+  if (op->fused) return B200_OK;  // no split-depth products
   // split-depth workspace: the widest summed weight gradient over the batch, four depth splits
   const size_t W = op->W, mn = std::max({W * 3, W * W, (size_t)op->H * W, (size_t)op->K * op->H});
   const size_t ws_len = std::max<size_t>(mn * (size_t)B * 4, (size_t)1 << 22);
