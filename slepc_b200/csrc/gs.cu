@@ -1046,7 +1046,9 @@ cudaError_t launch_column_t(ColumnParams &p, int G, cudaStream_t stream) {
   cfg.dynamicSmemBytes = stage * p.stages + 128;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeCooperative;  // the CTAs meet at grid barriers
+  // The CTAs meet at grid barriers: all of them are resident or none, also beside another stream's launches
+  // (columns and runs of two bases on two streams at once keep their bits).
+  attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
