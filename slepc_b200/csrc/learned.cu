@@ -55,7 +55,7 @@ struct b200_neural_op_s {
   float *mode_work = nullptr;      // modes_kernel: the blocks' shares and arrival counts
   unsigned *mode_count = nullptr;
   float *grad_part = nullptr;      // blocks' partial sums of the weight gradients
-  float2 *loss_part = nullptr, *loss_coef = nullptr;
+  float2 *loss_part = nullptr;
   float *hloss = nullptr;    // pinned: B x K losses, then the error word
   cudaEvent_t loss_ready = nullptr;
   float *ws = nullptr;       // split-depth partial products of the GEMMs
@@ -264,7 +264,7 @@ b200_status reserve(b200_neural_op op, int B) {
   op->loss_bk = nullptr;
   op->bias_part = op->grad_part = op->mode_work = nullptr;
   op->mode_count = nullptr;
-  op->loss_part = op->loss_coef = nullptr;
+  op->loss_part = nullptr;
   op->hloss = nullptr;
   op->cap = B;
   size_t len = 0;
@@ -280,7 +280,7 @@ b200_status reserve(b200_neural_op op, int B) {
              cudaSuccess &&
          cudaMalloc(&op->mode_count, sizeof(unsigned) * (size_t)B * op->W) == cudaSuccess &&
          cudaMemsetAsync(op->mode_count, 0, sizeof(unsigned) * (size_t)B * op->W, op->stream) == cudaSuccess &&
-         cudaMalloc(&op->loss_part, sizeof(float2) * BK * (slices + 1)) == cudaSuccess;
+         cudaMalloc(&op->loss_part, sizeof(float2) * BK * slices) == cudaSuccess;
   if (!ok) {
     cudaFree(op->act);
     op->act = nullptr;
@@ -288,7 +288,6 @@ b200_status reserve(b200_neural_op op, int B) {
     b200_set_last_error(__FILE__, __LINE__, "cudaMalloc failed for the neural-operator activations");
     return B200_ERR_NOMEM;
   }
-  if (op->fused) op->loss_coef = op->loss_part + BK * slices;
   op->act_len = len;
   if (op->fused) return B200_OK;  // no split-depth products
   // split-depth workspace: the widest summed weight gradient over the batch, four depth splits
@@ -567,13 +566,9 @@ b200_status loss_fused(b200_neural_op op, int B, const float *targets, const Act
   const int slices = (op->P + neural::kLossSlice - 1) / neural::kLossSlice, BK = B * op->K;
   neural::loss_part_kernel<<<dim3(slices, op->K, B), 256, 0, op->stream>>>(a.Y, targets, op->K, op->P, op->loss_part);
   count_launch();
-  neural::loss_final_kernel<<<(BK + 127) / 128, 128, 0, op->stream>>>(op->loss_part, slices, BK, 1.f / (float)BK, op->loss_bk,
-                                                                     op->loss_coef);
+  neural::loss_final_kernel<<<dim3(want_grad ? slices : 1, op->K, B), 256, 0, op->stream>>>(
+      op->loss_part, slices, op->K, op->P, 1.f / (float)BK, a.Y, targets, op->loss_bk, want_grad ? a.dY : nullptr);
   count_launch();
-  if (want_grad) {
-    neural::loss_grad_kernel<<<dim3(slices, op->K, B), 256, 0, op->stream>>>(a.Y, targets, op->loss_coef, op->K, op->P, a.dY);
-    count_launch();
-  }
   B200_CUDA_CHECK(cudaGetLastError());
   return loss_queue_read(op, B);
 }

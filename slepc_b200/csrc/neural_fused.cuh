@@ -361,33 +361,39 @@ __global__ void __launch_bounds__(256) loss_part_kernel(const float *__restrict_
     part[((size_t)b * K + k) * gridDim.x + blockIdx.x] = make_float2(yu, yy);
   }
 }
-// Second stage: loss_bk = 1 - (y.u)^2/(y.y) and the factors of dY = cu u + cy y.
-__global__ void loss_final_kernel(const float2 *__restrict__ part, int slices, int count, float scale, float *loss_bk,
-                                  float2 *coef) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= count) return;
+// Second stage: loss_bk = 1 - (y.u)^2/(y.y), and dY = cu u + cy y over the block's slice (dY null, one block per (k, b):
+// the loss alone).  Every block adds the slices' sums in their order for itself, which costs less than a launch between.
+// dY is formed here and not in the backward pass: once the loss can be read, no kernel reads the caller's targets.
+__global__ void __launch_bounds__(256) loss_final_kernel(const float2 *__restrict__ part, int slices, int K, int P,
+                                                         float scale, const float *__restrict__ Y,
+                                                         const float *__restrict__ T, float *loss_bk, float *dY) {
+  __shared__ float2 sums[256], coef;
+  const int e = blockIdx.z * K + blockIdx.y;
   float yu = 0.f, yy = 0.f;
-  for (int s = 0; s < slices; ++s) {
-    const float2 v = part[(size_t)e * slices + s];
-    yu += v.x;
-    yy += v.y;
+  for (int s0 = 0; s0 < slices; s0 += 256) {
+    if (s0 + (int)threadIdx.x < slices) sums[threadIdx.x] = __ldg(part + (size_t)e * slices + s0 + threadIdx.x);
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll 8
+      for (int s = 0; s < min(256, slices - s0); ++s) {
+        yu += sums[s].x;
+        yy += sums[s].y;
+      }
+    __syncthreads();
   }
-  yy = fmaxf(yy, 1e-30f);
-  loss_bk[e] = 1.f - yu * yu / yy;
-  coef[e] = make_float2(-2.f * yu / yy * scale, 2.f * yu * yu / (yy * yy) * scale);
-}
-
-// dY = cu T + cy Y over the slices of loss_part_kernel.  A kernel of its own, before the loss is read back, so that
-// no later kernel reads the caller's targets.
-__global__ void __launch_bounds__(256) loss_grad_kernel(const float *__restrict__ Y, const float *__restrict__ T,
-                                                        const float2 *__restrict__ coef, int K, int P, float *dY) {
-  const int k = blockIdx.y, b = blockIdx.z;
-  const size_t base = ((size_t)b * K + k) * P;
-  const float2 cf = __ldg(coef + b * K + k);
+  if (threadIdx.x == 0) {
+    yy = fmaxf(yy, 1e-30f);
+    if (blockIdx.x == 0) loss_bk[e] = 1.f - yu * yu / yy;
+    coef = make_float2(-2.f * yu / yy * scale, 2.f * yu * yu / (yy * yy) * scale);
+  }
+  if (!dY) return;
+  __syncthreads();
+  const size_t base = (size_t)e * P;
+  const float cu = coef.x, cy = coef.y;
   const int p1 = min(P, (int)(blockIdx.x + 1) * kLossSlice);
 #pragma unroll 4
   for (int p = blockIdx.x * kLossSlice + threadIdx.x; p < p1; p += 256)
-    dY[base + p] = cf.x * __ldg(T + base + p) + cf.y * __ldg(Y + base + p);
+    dY[base + p] = cu * __ldg(T + base + p) + cy * __ldg(Y + base + p);
 }
 
 // Projection, backward: dH = Q2^T dY, dZ = dH gelu'(Z) (written for the gradient of Q1), dV = Q1^T dZ for at most 32
