@@ -454,7 +454,9 @@ typedef struct {
   int64_t spmm_columns;
 } b200_eps_stats;
 b200_status b200_eps_get_stats(b200_eps eps, b200_eps_stats *stats);
-/* Enable per-phase CUDA-event timing (adds events around each phase). */
+/* Enable per-phase CUDA-event timing (adds events around each phase).  A timed solve launches its
+ * products and Gram-Schmidt columns one by one, so where the plain solve runs a whole Lanczos run in
+ * one launch (small bases), ms_orth and ms_spmv are those of the separate launches. */
 b200_status b200_eps_set_timing(b200_eps eps, int on);
 
 /* EPSMonitorSet (src/eps/interface/epsmon.c:96) / EPSMonitorCancel: a monitor

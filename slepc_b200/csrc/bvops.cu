@@ -406,9 +406,10 @@ __device__ __forceinline__ void dmma_m16n8k16(double (&d)[4], const double (&a)[
 // through a ring of kGramStages stages of 32 rows with asynchronous copies (column stride 36 doubles, 4 mod 16: the
 // fragment loads of a half warp hit distinct banks).  Warps 0..3 take the first 16 rows of a stage and warps 4..7 the
 // others, each a quarter of the products of the 16-column strips of Y (STRIPS) with the 8-column tiles of X, so that
-// the four schedulers have the same share; the row halves meet in shared memory at the end.  SELF: X is Y, staged once.  Fragments (g = lane / 4, t = lane % 4): A = Y^T, element e
-// at row g + 8 (e % 2), depth t + 4 (e / 2); B element e at depth t + 4 e, column g; D element e at row
-// g + 8 (e / 2), column 2 t + e % 2.  partial[cta * nx ny + i + j ny].
+// the four schedulers have the same share; the row halves meet in shared memory at the end.  SELF: X is Y, staged
+// once.  Fragments (g = lane / 4, t = lane % 4): A = Y^T, element e at row g + 8 (e % 2), depth t + 4 (e / 2); B
+// element e at depth t + 4 e, column g; D element e at row g + 8 (e / 2), column 2 t + e % 2.
+// partial[cta * nx ny + i + j ny].
 //
 // Bound: for 48 x 48 columns of n = 262,144 rows 201 MB (31 us) and 1.2 GFLOP (33 us at the 37 TFLOP/s of this
 // shape).  A whole b200_bv_dot of that size takes 97 us with its read-back (110 us with a strip per warp, which leaves
@@ -1154,7 +1155,11 @@ cudaError_t dot_launch(const double *X, int ldx, int nx, const double *Y, int ld
     const int strips = ny > 48 ? 4 : (ny + 15) / 16;
     cudaError_t e;
     switch (strips) {
-#define B200_GRAM_CASE(S)                                                                                         case S:                                                                                                           e = self ? gram_mma_launch<S, true>(X, ldx, nx, Y, ldy, ny, n, work, blocks, stream)                                     : gram_mma_launch<S, false>(X, ldx, nx, Y, ldy, ny, n, work, blocks, stream);                          break;
+#define B200_GRAM_CASE(S)                                                                         \
+  case S:                                                                                         \
+    e = self ? gram_mma_launch<S, true>(X, ldx, nx, Y, ldy, ny, n, work, blocks, stream)          \
+             : gram_mma_launch<S, false>(X, ldx, nx, Y, ldy, ny, n, work, blocks, stream);        \
+    break;
       B200_GRAM_CASE(1)
       B200_GRAM_CASE(2)
       B200_GRAM_CASE(3)

@@ -10,8 +10,8 @@
 namespace b200 {
 
 // Largest number of basis columns a BV may hold (ncv+1 plus the internal
-// work column).  Bounded by the per-CTA column accumulators of the
-// Gram-Schmidt kernels (one per thread of a 256-thread block).
+// work column).  A Gram-Schmidt CTA holds 8 warps x 32 columns a lane, and a
+// tile load's box has at most 256 columns.
 constexpr int kMaxCols = 255;
 
 // Number of spin iterations after which a device-side wait gives up.

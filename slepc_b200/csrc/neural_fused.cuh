@@ -8,7 +8,7 @@
 // each reads its two fields once, and one kernel adds the blocks' sums of all of them.
 //
 // Measured (loss and gradients, width 32, 16 modes, 4 layers): 512 x 512 grid, batch 4, 12.2 ms as separate
-// products and elementwise kernels (113 launches), 3.6 ms so (38 launches); 64 x 64 grid, batch 16, 1.58 -> 0.84 ms.
+// products and elementwise kernels (113 launches), 3.5 ms so (38 launches); 64 x 64 grid, batch 16, 1.56 -> 0.85 ms.
 #pragma once
 #include "common.h"
 
